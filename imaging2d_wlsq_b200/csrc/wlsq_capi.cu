@@ -2,6 +2,7 @@
 // reference-compatible entry points.  Declarations and contracts: include/imaging2d_wlsq_b200.h.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <map>
 #include <cstdio>
 #include <cstdlib>
@@ -16,6 +17,7 @@
 #include "wlsq_kernels.cuh"
 #include "wlsq_cluster.cuh"
 #include "wlsq_cluster2.cuh"
+#include "wlsq_rows.cuh"
 #include "wlsq_wide.cuh"
 #include "wlsq_adjoint.cuh"
 #include "wlsq_adjoint_cluster.cuh"
@@ -73,6 +75,60 @@ static KernelFn find_fixed(int G, int L)
     for (const auto &k : kFixed)
         if (k.G == G && k.L == L) return k.fn;
     return nullptr;
+}
+
+// Row-split kernels by slots per item, tap pairs per lane and number of tables; 4 outputs per quad.
+// One slot keeps its rows' next taps in registers (the row loads are its whole traffic: 3.36 against
+// 3.76 ms for one shot of 1024 x 500, 256 frequencies, 31 taps); with two slots those registers are
+// better left to the second slot (32 shots, two tables: 3.2 against 4.2 ms with one slot an item).
+// Tried on the same cases and slower: 8 outputs per quad with one slot (3.58 ms, 168 registers, and
+// 3.45 without the held taps), three CTAs per SM at 80 registers (3.76), 4 slots per item (spills).
+struct RowsKernel {
+    int G, np;
+    bool two;
+    KernelFn fn;
+};
+#define IMG2D_ROWS(G, NP, PIPE) \
+    {G, NP, false, migrate_rows_kernel<G, NP, false, PIPE>}, {G, NP, true, migrate_rows_kernel<G, NP, true, PIPE>}
+#define IMG2D_ROWS_NP(G, PIPE)                                                                            \
+    IMG2D_ROWS(G, 1, PIPE), IMG2D_ROWS(G, 2, PIPE), IMG2D_ROWS(G, 3, PIPE), IMG2D_ROWS(G, 4, PIPE),       \
+        IMG2D_ROWS(G, 5, PIPE), IMG2D_ROWS(G, 6, PIPE), IMG2D_ROWS(G, 7, PIPE), IMG2D_ROWS(G, 8, PIPE),   \
+        IMG2D_ROWS(G, 10, PIPE)
+static const RowsKernel kRows[] = {IMG2D_ROWS_NP(1, true), IMG2D_ROWS_NP(2, false)};
+
+static KernelFn find_rows(int G, int L, bool two)
+{
+    if (L < 3) return nullptr;
+    for (const auto &k : kRows)
+        if (k.G == G && k.np == rows_np(L) && k.two == two) return k.fn;
+    return nullptr;
+}
+
+// Threads per CTA and estimated time of the row-split kernel, in microseconds per depth step, for
+// n_items items of windows up to W.  A step of a CTA is `rounds` blocks per warp, each taking
+// 0.45 us (1 + k / 6) with k warps on the SM, times 1.45 for two slots (fitted on a B200, 31 taps,
+// one table: 3 to 16 warps per SM; within 15% on the cases it was checked on); items beyond what is
+// resident run in further waves.
+struct RowsLaunch {
+    int warps;
+    double us;
+};
+static RowsLaunch rows_launch(int G, int W, int L, bool two, long long n_items, int nsm, size_t smem_sm)
+{
+    const int nwb = (W + kRowsWarpPos - 1) / kRowsWarpPos;
+    const size_t smem = rows_smem_bytes(G, W, L) + 1024;
+    RowsLaunch best{1, 1e30};
+    for (int w = 1; w <= std::min(nwb, kRowsThreads / 32); ++w) {
+        const long long c = std::min<long long>(16 / w, (long long)(smem_sm / smem));  // 128 registers a thread
+        if (c < 1) continue;
+        const int rounds = (nwb + w - 1) / w;
+        auto wave = [&](long long per_sm) { return rounds * 0.45 * (1.0 + per_sm * w / 6.0); };
+        const long long full = n_items / (nsm * c), rest = n_items % (nsm * c);
+        double us = full * wave(c) + (rest ? wave((rest + nsm - 1) / nsm) : 0.0);
+        us *= (G == 2 ? 1.45 : 1.0) * (two ? 1.2 : 1.0) * (0.25 + 0.75 * rows_np(L) / 4);
+        if (us < best.us) best = RowsLaunch{w, us};
+    }
+    return best;
 }
 
 static KernelFn find_generic(int G, int mode)
@@ -429,13 +485,15 @@ struct img2d_plan {
     std::vector<int> group_order;  // migration groups, widest first (the order of the item queue)
     int cluster = 0;  // CTAs per cluster of the cluster kernel, 0 = single-CTA kernels
     int block = 256;                  // threads per CTA of the chosen kernel
+    bool allow_rows = true;
+    bool rows = false;                // the row-split kernel (its table order, visit counts per CTA)
     int variant = -1;                 // index into the cluster2 variant table
     int tab16 = 0;                    // operator table storage: 0 FP32, 1 FP16, 2 BF16
     const char *kname = "";           // name of the chosen kernel
     img2d::Carver *carver = nullptr;  // no-allocation mode: buffers carved from fixed scratch
     cudaStream_t upload_stream = 0;   // no-allocation mode: stream of the descriptor uploads
     bool timing = true;               // record events around the migration kernel
-    img2d::DevBuf items, groups, segs, owner, shot_off, idx, tabF, tabB, tab16buf, partial, comp, counter, naive_buf;
+    img2d::DevBuf items, groups, segs, owner, shot_off, idx, tabF, tabB, tab16buf, tab_rows, partial, comp, visits, counter, naive_buf;
     // dense tables (drop-in ABI) are owned by the caller of run_dense
     // lane-slot packing: shots of each slot, slots ordered by extent, right end of each slot
     std::vector<std::vector<int>> slots;
@@ -926,6 +984,9 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         return fail(IMG2D_EINVAL, "IMG2D_FLAG_WIDE_BULK runs packed FMAs; it does not combine with "
                                   "IMG2D_FLAG_WIDE_SCALAR");
     const bool wide_requested = (flags & wide_flags) != 0;
+    const bool explicit_kernel = wide_requested || explicit_variant || tab16 ||
+                                 (flags & (IMG2D_FLAG_GENERIC | IMG2D_FLAG_NO_CLUSTER | IMG2D_FLAG_CLUSTER_V1 |
+                                           IMG2D_FLAG_CLUSTER2 | IMG2D_FLAG_LINE_PACKING)) != 0;
     const bool wide_ok = mode == OP_CONJ && !tab16 && p->L >= 7 &&
                          !(flags & (IMG2D_FLAG_GENERIC | IMG2D_FLAG_NO_CLUSTER | IMG2D_FLAG_CLUSTER_V1 |
                                     IMG2D_FLAG_CLUSTER2)) &&
@@ -942,8 +1003,42 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                              : 0;
         want_wide = p->n_slots < 12 || busy < nsm * 96 / 100;
     }
-    if (want_wide) try_wide();
-    if (!p->cluster && cluster_ok && !(flags & (IMG2D_FLAG_CLUSTER_V1 | wide_flags)) &&
+    // The row-split kernel instead: always for a table pair, and for single tables where it is
+    // estimated faster than the kernel chosen below.  Surveys of 12 slots or more are only considered
+    // when its items fill the SMs (the estimates are made for that).
+    int rows_G = 1;
+    RowsLaunch rows_l{1, 1e30};
+    if (p->allow_rows && mode != OP_DENSE && !explicit_kernel && find_rows(1, p->L, mode == OP_TWO)) {
+        int smem_sm = 0;
+        IMG2D_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+        for (int G = 1; G <= std::min(2, p->n_slots); ++G) {
+            const int widest = make_groups(G);
+            if (rows_smem_bytes(G, widest, p->L) + static_reserve > (size_t)smem_optin) continue;
+            const long long n = (long long)groups.size() * nf;
+            if (p->n_slots >= 12 && mode == OP_CONJ && n < nsm) continue;
+            const RowsLaunch r = rows_launch(G, widest, p->L, mode == OP_TWO, n, nsm, smem_sm);
+            if (r.us < rows_l.us) {
+                rows_l = r;
+                rows_G = G;
+            }
+        }
+        if (rows_l.us < 1e30) {
+            if (mode == OP_TWO || p->n_slots < 6) {
+                p->rows = true;
+            } else {
+                // wide kernel: 8 slots x up to 1024 positions per CTA; cluster2: 16 x 512
+                const bool wide = want_wide;
+                const int G = wide ? WideShape::G : 16, pc = wide ? WideShape::PC : 512;
+                const int widest = make_groups(G), K = (widest + pc - 1) / pc;
+                const int nc = wide ? std::min(pc, (widest + K * 256 - 1) / (K * 256) * 256) : pc;
+                const double item = (wide ? wide_item_cost(nc, 1) * 17.0 : 17.0) * (p->L + 5) / 40.0;
+                const double waves = (double)groups.size() * nf * K / nsm;
+                p->rows = rows_l.us < 0.95 * item * (waves <= 4.0 ? std::ceil(waves) : waves + 0.5);
+            }
+        }
+    }
+    if (!p->rows && want_wide) try_wide();
+    if (!p->cluster && !p->rows && cluster_ok && !(flags & (IMG2D_FLAG_CLUSTER_V1 | wide_flags)) &&
         p->L >= 7) {
         // the default ring variant needs 33 KB more shared memory than the staged one: long
         // operators or very wide windows fall back to the staged variant
@@ -955,7 +1050,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                                   "window <= 16 CTAs)");
     p->tab16 = tab16;
     const ClusterKernel *ck = cluster_ok ? find_cluster(p->L) : nullptr;
-    if (!p->cluster && ck && ck->smem + static_reserve <= (size_t)smem_optin) {
+    if (!p->cluster && !p->rows && ck && ck->smem + static_reserve <= (size_t)smem_optin) {
         const int widest = make_groups(ClusterShape::G);
         const int K = (widest + ClusterShape::PC - 1) / ClusterShape::PC;
         if (K <= 8) {
@@ -968,7 +1063,17 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             p->kname = "migrate_cluster";
         }
     }
-    if (!p->cluster) {
+    if (p->rows) {
+        p->cluster = 0;
+        p->G = rows_G;
+        p->fixed = true;
+        p->fn = find_rows(rows_G, p->L, mode == OP_TWO);
+        p->max_w = make_groups(rows_G);
+        p->smem = rows_smem_bytes(rows_G, p->max_w, p->L);
+        p->block = 32 * rows_l.warps;
+        p->kname = "migrate_rows";
+    }
+    if (!p->cluster && !p->rows) {
         int nsp2 = 1;
         while (nsp2 < p->n_slots) nsp2 <<= 1;
         int G = 8;
@@ -1026,11 +1131,31 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         IMG2D_CUDA(cudaOccupancyMaxActiveClusters(&nclusters, (void *)p->fn, &cfg));
         if (nclusters <= 0) return fail(IMG2D_ECUDA, "no cluster of this size fits on the device");
         p->grid = std::min(p->n_items, nclusters) * p->cluster;
+    } else if (p->rows) {
+        int per_sm = 0;
+        IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->fn, p->block, p->smem));
+        if (per_sm <= 0) return fail(IMG2D_ECUDA, "the row-split kernel does not fit on an SM");
+        p->grid = std::min(p->n_items, nsm * per_sm);
     } else {
         p->grid = std::min(p->n_items, nsm);
     }
 
     int rc;
+    const size_t plane = (size_t)nextrap * nx;
+    const size_t rows_tab_b = p->rows ? (size_t)nk * rows_row_floats(p->L, mode == OP_TWO) * sizeof(float) : 0;
+    if (p->carver && p->rows) {
+        // fixed scratch: the row-split kernel only where the partial images of all its CTAs fit
+        const size_t need = items.size() * sizeof(int2) + groups.size() * sizeof(GroupDesc) +
+                            segs.size() * sizeof(int4) + owner.size() * sizeof(int16_t) +
+                            p->off.size() * sizeof(long long) + (size_t)p->grid * sizeof(int) +
+                            (size_t)nf * nextrap * ((nx + 7) / 8 * 8) * sizeof(uint16_t) + rows_tab_b +
+                            (size_t)nk * ((p->L + 1) / 2 * 2) * sizeof(cpx) * (mode == OP_TWO ? 2 : 1) +
+                            (size_t)p->grid * plane * sizeof(float) * (p->n_items > p->grid ? 2 : 1) + 16 * 256;
+        if (need > p->carver->cap - p->carver->used) {
+            p->allow_rows = p->rows = false;
+            return build_plan(p, ns, nextrap, nz, nx, nf, nt, M, nk, shot_x0, shot_nx, flags, mode);
+        }
+    }
     if ((rc = p->items.ensure(items.size() * sizeof(int2)))) return rc;
     if ((rc = p->groups.ensure(groups.size() * sizeof(GroupDesc)))) return rc;
     if ((rc = p->segs.ensure(segs.size() * sizeof(int4)))) return rc;
@@ -1054,8 +1179,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         IMG2D_CUDA(cudaMemcpy(p->owner.p, owner.data(), owner.size() * sizeof(int16_t), cudaMemcpyHostToDevice));
         IMG2D_CUDA(cudaMemcpy(p->shot_off.p, p->off.data(), p->off.size() * sizeof(long long), cudaMemcpyHostToDevice));
     }
-    const size_t plane = (size_t)nextrap * nx;
-    if (p->carver) {
+    if (p->carver && !p->rows) {
         // fixed scratch: fewer persistent CTAs when their private image partials would not fit
         const size_t idx_b = (size_t)nf * nextrap * ((nx + 7) / 8 * 8) * sizeof(uint16_t) + 256;
         const size_t tab_b = ((size_t)nk * ((p->L + 1) / 2 * 2) * sizeof(cpx) + 256) * (mode == OP_TWO ? 2 : 1);
@@ -1067,8 +1191,16 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                                           " MiB of fixed scratch of the no-allocation entry point");
         p->grid = (int)std::min<size_t>((size_t)p->grid, fit);
     }
-    if ((rc = p->partial.ensure((size_t)p->grid * plane * sizeof(float)))) return rc;
-    if ((rc = p->comp.ensure((size_t)p->grid * plane * sizeof(float)))) return rc;
+    for (;;) {
+        rc = p->partial.ensure((size_t)p->grid * plane * sizeof(float));
+        if (!rc && (!p->rows || p->n_items > p->grid))  // one item per CTA needs no compensation
+            rc = p->comp.ensure((size_t)p->grid * plane * sizeof(float));
+        if (!rc) break;
+        // the row-split kernel has several CTAs per SM: with less memory it runs on fewer
+        if (rc != IMG2D_ENOMEM || !p->rows || p->grid <= 1) return rc;
+        p->partial.release();
+        p->grid = p->grid > nsm ? std::max(nsm, p->grid / 2) : p->grid / 2;
+    }
     if (mode != OP_DENSE) {
         p->idx_lstride = (nx + 7) / 8 * 8;
         if ((rc = p->idx.ensure((size_t)nf * nextrap * p->idx_lstride * sizeof(uint16_t)))) return rc;
@@ -1076,6 +1208,10 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         if ((rc = p->tabF.ensure((size_t)nk * p->tab_stride * sizeof(cpx)))) return rc;
         if (p->tab16 && (rc = p->tab16buf.ensure((size_t)nk * p->tab_stride * sizeof(unsigned)))) return rc;
         if (mode == OP_TWO && (rc = p->tabB.ensure((size_t)nk * p->tab_stride * sizeof(cpx)))) return rc;
+    }
+    if (p->rows) {
+        if ((rc = p->visits.ensure((size_t)p->grid * sizeof(int)))) return rc;
+        if ((rc = p->tab_rows.ensure(rows_tab_b))) return rc;
     }
     return IMG2D_OK;
 }
@@ -1097,6 +1233,12 @@ static MigrateArgs base_args(img2d_plan *p, cpx *wave, cpx *shot)
     a.tabF = p->tabF.as<cpx>();
     a.tabB = p->mode == OP_TWO ? p->tabB.as<cpx>() : p->tabF.as<cpx>();
     a.tab16 = p->tab16buf.p;
+    if (p->rows) {
+        a.tab_rows = p->tab_rows.p;
+        const RowsStarts rs = rows_starts(p->L);
+        for (int i = 0; i < 4; ++i) a.row_start[i] = rs.s[i];
+        a.row_apart = rs.apart;
+    }
     a.idx = p->idx.as<uint16_t>();
     a.idx_jstride = (long long)p->nextrap * p->idx_lstride;
     a.idx_lstride = p->idx_lstride;
@@ -1137,7 +1279,7 @@ static int launch_kernel(img2d_plan *p, const MigrateArgs &a, int grid, cudaStre
         cfg.numAttrs = 1;
         IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->fn, a));
     } else {
-        p->fn<<<grid, 256, p->smem, st>>>(a);
+        p->fn<<<grid, p->block, p->smem, st>>>(a);
     }
     IMG2D_CUDA(cudaGetLastError());
     return IMG2D_OK;
@@ -1151,7 +1293,12 @@ static int launch(img2d_plan *p, MigrateArgs a, float *d_image, float *d_image_s
     IMG2D_CUDA(cudaMemsetAsync(p->counter.p, 0, 2 * sizeof(int), st));
     a.status = p->counter.as<int>() + 1;
     p->launched = true;
-    if (d_image) {
+    if (d_image && p->rows) {
+        IMG2D_CUDA(cudaMemsetAsync(p->visits.p, 0, (size_t)p->grid * sizeof(int), st));
+        a.partial = p->partial.as<float>();
+        a.comp = p->comp.as<float>();
+        a.visits = p->visits.as<int>();
+    } else if (d_image) {
         IMG2D_CUDA(cudaMemsetAsync(p->partial.p, 0, (size_t)p->grid * plane * sizeof(float), st));
         IMG2D_CUDA(cudaMemsetAsync(p->comp.p, 0, (size_t)p->grid * plane * sizeof(float), st));
         a.partial = p->partial.as<float>();
@@ -1175,8 +1322,8 @@ static int launch(img2d_plan *p, MigrateArgs a, float *d_image, float *d_image_s
         p->ev_recorded = true;
     }
     if (d_image) {
-        const int blocks = (int)std::min<size_t>((plane + 255) / 256, 148 * 8);
-        reduce_partials_kernel<<<blocks, 256, 0, st>>>(p->partial.as<float>(), p->comp.as<float>(), p->grid,
+        const int blocks = (int)std::min<size_t>((plane + 31) / 32, 148 * 64);
+        reduce_partials_kernel<<<blocks, 256, 0, st>>>(p->partial.as<float>(), p->comp.as<float>(), a.visits, p->grid,
                                                        (long long)plane, d_image);
         IMG2D_CUDA(cudaGetLastError());
     }
@@ -1196,6 +1343,13 @@ static int set_model(img2d_plan *p, const double *d_omega, const double *d_vel, 
     if (p->mode == OP_TWO) {
         IMG2D_CUDA(cudaMemsetAsync(p->tabB.p, 0, (size_t)p->nk * prow, st));
         IMG2D_CUDA(cudaMemcpy2DAsync(p->tabB.p, prow, d_tabB, row, row, p->nk, cudaMemcpyDeviceToDevice, st));
+    }
+    if (p->rows) {
+        const long long n = (long long)p->nk * rows_row_floats(p->L, p->mode == OP_TWO) / 2;
+        rows_table_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(
+            d_tabF, p->mode == OP_TWO ? d_tabB : nullptr, p->L, rows_np(p->L), rows_starts(p->L),
+            p->nk, p->tab_rows.as<float>());
+        IMG2D_CUDA(cudaGetLastError());
     }
     if (p->tab16) {
         const long long n = (long long)p->nk * p->tab_stride;
@@ -1474,6 +1628,7 @@ static int migrate_chunked(img2d_plan *p, HostEntryBuffers &hb, int C, img2d_c64
     if ((rc = p->partial.ensure(2 * set_bytes))) return rc;
     if ((rc = p->comp.ensure(2 * set_bytes))) return rc;
     if ((rc = hb.pipe_counter.ensure(4 * sizeof(int)))) return rc;
+    if (p->rows && (rc = p->visits.ensure(2 * (size_t)p->grid * sizeof(int)))) return rc;
     for (cudaStream_t &x : hb.st)
         if (!x) IMG2D_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
     while ((int)hb.ev.size() < 2 * C + 1) {
@@ -1485,8 +1640,12 @@ static int migrate_chunked(img2d_plan *p, HostEntryBuffers &hb, int C, img2d_c64
     int *cnt = hb.pipe_counter.as<int>();
     float *part = p->partial.as<float>(), *comp = p->comp.as<float>();
     // zeroed partial sets, counters and status words before the first launch of either stream
-    IMG2D_CUDA(cudaMemsetAsync(part, 0, 2 * set_bytes, sk[0]));
-    IMG2D_CUDA(cudaMemsetAsync(comp, 0, 2 * set_bytes, sk[0]));
+    if (p->rows) {
+        IMG2D_CUDA(cudaMemsetAsync(p->visits.p, 0, 2 * (size_t)p->grid * sizeof(int), sk[0]));
+    } else {
+        IMG2D_CUDA(cudaMemsetAsync(part, 0, 2 * set_bytes, sk[0]));
+        IMG2D_CUDA(cudaMemsetAsync(comp, 0, 2 * set_bytes, sk[0]));
+    }
     IMG2D_CUDA(cudaMemsetAsync(cnt, 0, 4 * sizeof(int), sk[0]));
     IMG2D_CUDA(cudaEventRecord(hb.ev[2 * C], sk[0]));
     IMG2D_CUDA(cudaStreamWaitEvent(sk[1], hb.ev[2 * C], 0));
@@ -1520,6 +1679,7 @@ static int migrate_chunked(img2d_plan *p, HostEntryBuffers &hb, int C, img2d_c64
         a.status = cnt + 2 + (c & 1);
         a.partial = dI ? part + (size_t)(c & 1) * p->grid * plane : nullptr;
         a.comp = dI ? comp + (size_t)(c & 1) * p->grid * plane : nullptr;
+        a.visits = dI && p->rows ? p->visits.as<int>() + (size_t)(c & 1) * p->grid : nullptr;
         if ((rc = launch_kernel(p, a, std::min(n, p->grid / K) * K, st))) return rc;
         IMG2D_CUDA(cudaEventRecord(hb.ev[2 * c + 1], st));
         if (c >= 1) {
@@ -1532,8 +1692,9 @@ static int migrate_chunked(img2d_plan *p, HostEntryBuffers &hb, int C, img2d_c64
     if (dI) {
         IMG2D_CUDA(cudaStreamWaitEvent(sk[0], hb.ev[2 * C - 1], 0));
         if (C >= 2) IMG2D_CUDA(cudaStreamWaitEvent(sk[0], hb.ev[2 * C - 3], 0));
-        const int blocks = (int)std::min<size_t>((plane + 255) / 256, 148 * 8);
-        reduce_partials_kernel<<<blocks, 256, 0, sk[0]>>>(part, comp, 2 * p->grid, (long long)plane, dI);
+        const int blocks = (int)std::min<size_t>((plane + 31) / 32, 148 * 64);
+        reduce_partials_kernel<<<blocks, 256, 0, sk[0]>>>(part, comp, p->rows ? p->visits.as<int>() : nullptr, 2 * p->grid,
+                                                          (long long)plane, dI);
         IMG2D_CUDA(cudaGetLastError());
     }
     for (cudaStream_t x : hb.st) IMG2D_CUDA(cudaStreamSynchronize(x));
