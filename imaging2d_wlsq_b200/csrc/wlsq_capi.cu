@@ -21,6 +21,7 @@
 #include "wlsq_wide.cuh"
 #include "wlsq_adjoint.cuh"
 #include "wlsq_adjoint_cluster.cuh"
+#include "wlsq_rows_adjoint.cuh"
 #include "wlsq_frontend.cuh"
 
 namespace img2d {
@@ -218,6 +219,25 @@ static DemigFn find_demig_cluster(int L, bool ring = false)
         if (k.L == 0) generic = k.fn;
     }
     return ring ? nullptr : generic;
+}
+
+// Row-split demigration kernels by slots per item and tap pairs per lane.
+struct DemigRowsKernel {
+    int NS, np;
+    void (*fn)(RowsAdjArgs);
+};
+#define IMG2D_DROWS(NP) {1, NP, demigrate_rows_kernel<1, NP>}, {2, NP, demigrate_rows_kernel<2, NP>}
+static const DemigRowsKernel kDemigRows[] = {
+    IMG2D_DROWS(1), IMG2D_DROWS(2), IMG2D_DROWS(3), IMG2D_DROWS(4), IMG2D_DROWS(5),
+    IMG2D_DROWS(6), IMG2D_DROWS(7), IMG2D_DROWS(8), IMG2D_DROWS(10),
+};
+
+static void (*find_demig_rows(int NS, int L))(RowsAdjArgs)
+{
+    if (L < 3) return nullptr;
+    for (const auto &k : kDemigRows)
+        if (k.NS == NS && k.np == rows_np(L)) return k.fn;
+    return nullptr;
 }
 
 static DemigFn find_demig(int G, int L)
@@ -485,7 +505,7 @@ struct img2d_plan {
     std::vector<int> group_order;  // migration groups, widest first (the order of the item queue)
     int cluster = 0;  // CTAs per cluster of the cluster kernel, 0 = single-CTA kernels
     int block = 256;                  // threads per CTA of the chosen kernel
-    bool allow_rows = true;
+    bool allow_rows = true, rows_tab_set = false;
     bool rows = false;                // the row-split kernel (its table order, visit counts per CTA)
     int variant = -1;                 // index into the cluster2 variant table
     int tab16 = 0;                    // operator table storage: 0 FP32, 1 FP16, 2 BF16
@@ -501,6 +521,9 @@ struct img2d_plan {
     // demigration (adjoint) launch state, built on its first call
     int adj_G = 0, adj_grid = 0, adj_items_n = 0, adj_wmax = 0, adj_block = 0, adj_slab = 0, adj_nslab = 0;
     int adj_cluster = 0;               // CTAs per cluster of the cluster demigration kernel, 0 = single CTA
+    bool adj_rows = false, adj_allow_rows = true;  // the row-split demigration kernel
+    void (*adj_rows_fn)(img2d::RowsAdjArgs) = nullptr;
+    bool adj_full_cache = false;       // kept source: every depth step of every item (else per-CTA planes only)
     bool adj_ring = false;             // its forward steps read operator pairs through the shared-memory ring
     bool model_set = false;            // set_model has built the padded tables and the operator index
     long long adj_work_cta = 0, adj_cache_item = 0;  // float2 elements: per-CTA work area, kept per item
@@ -1330,6 +1353,21 @@ static int launch(img2d_plan *p, MigrateArgs a, float *d_image, float *d_image_s
     return IMG2D_OK;
 }
 
+// The row-split kernels' copy of the plan's tables.
+static int set_rows_table(img2d_plan *p, cudaStream_t st)
+{
+    const bool two = p->mode == OP_TWO;
+    const long long floats = (long long)p->nk * rows_row_floats(p->L, two);
+    const int rc = p->tab_rows.ensure((size_t)floats * sizeof(float));
+    if (rc) return rc;
+    rows_table_kernel<<<(int)std::min<long long>((floats / 2 + 255) / 256, 148 * 8), 256, 0, st>>>(
+        p->tabF.as<cpx>(), two ? p->tabB.as<cpx>() : nullptr, p->tab_stride, p->L, rows_np(p->L), rows_starts(p->L),
+        p->nk, p->tab_rows.as<float>());
+    IMG2D_CUDA(cudaGetLastError());
+    p->rows_tab_set = true;
+    return IMG2D_OK;
+}
+
 static int set_model(img2d_plan *p, const double *d_omega, const double *d_vel, double dk,
                      const cpx *d_tabF, const cpx *d_tabB, cudaStream_t st)
 {
@@ -1344,12 +1382,10 @@ static int set_model(img2d_plan *p, const double *d_omega, const double *d_vel, 
         IMG2D_CUDA(cudaMemsetAsync(p->tabB.p, 0, (size_t)p->nk * prow, st));
         IMG2D_CUDA(cudaMemcpy2DAsync(p->tabB.p, prow, d_tabB, row, row, p->nk, cudaMemcpyDeviceToDevice, st));
     }
+    p->rows_tab_set = false;
     if (p->rows) {
-        const long long n = (long long)p->nk * rows_row_floats(p->L, p->mode == OP_TWO) / 2;
-        rows_table_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(
-            d_tabF, p->mode == OP_TWO ? d_tabB : nullptr, p->L, rows_np(p->L), rows_starts(p->L),
-            p->nk, p->tab_rows.as<float>());
-        IMG2D_CUDA(cudaGetLastError());
+        const int rc = set_rows_table(p, st);
+        if (rc) return rc;
     }
     if (p->tab16) {
         const long long n = (long long)p->nk * p->tab_stride;
@@ -1366,6 +1402,11 @@ static int set_model(img2d_plan *p, const double *d_omega, const double *d_vel, 
     return IMG2D_OK;
 }
 
+// Row-split demigration: the kept source of all items takes at most this many complex values (8 GB);
+// above, IMG2D_SOURCE_KEEP keeps nothing of use and every call steps the source again, which costs
+// what the slab recomputation from kept checkpoints costs the other kernels.
+constexpr long long kDemigRowsCacheElems = 1ll << 30;
+
 // Launch state of the demigration: its own slot groups (one complex wavefield per slot, so up to
 // 8 slots fit beside the halos), items, and the per-CTA checkpoint / slab / save planes.
 static int demig_prepare(img2d_plan *p, int slab)
@@ -1373,7 +1414,7 @@ static int demig_prepare(img2d_plan *p, int slab)
     if (slab <= 0) slab = 8;
     slab = std::min(slab, p->nextrap);
     const int nslab = (p->nextrap + slab - 1) / slab;
-    if (p->adj_fn && p->adj_slab == slab) return IMG2D_OK;
+    if ((p->adj_fn || p->adj_rows_fn) && p->adj_slab == slab) return IMG2D_OK;
     p->adj_cache_valid = false;  // the checkpoint layout depends on the slab depth
     int dev = 0, smem_optin = 0, nsm = 0;
     IMG2D_CUDA(cudaGetDevice(&dev));
@@ -1407,7 +1448,17 @@ static int demig_prepare(img2d_plan *p, int slab)
             try_fn(find_demig_cluster(p->L, true), demigc_ring_smem_bytes(p->M), true);
         try_fn(find_demig_cluster(p->L), demigc_smem_bytes(p->M), false);
     }
-    if (!K) {
+    // Fewer slots: the row-split kernel, which keeps every S_l, where its shared memory fits.
+    void (*rows_fn)(RowsAdjArgs) = nullptr;
+    if (!K && p->adj_allow_rows && p->n_slots < 12 && !(p->flags & (IMG2D_FLAG_NO_CLUSTER | IMG2D_FLAG_GENERIC))) {
+        for (G = p->n_slots >= 2 ? 2 : 1; G >= 1 && !rows_fn; --G) {
+            widest = pack_groups(p, G, groups, segs, owner);
+            smem = rows_adj_smem_bytes(G, widest, p->L);
+            if (smem + static_reserve <= (size_t)smem_optin) rows_fn = find_demig_rows(G, p->L);
+        }
+        G = rows_fn ? G + 1 : 8;
+    }
+    if (!K && !rows_fn) {
         for (;; G >>= 1) {
             widest = pack_groups(p, G, groups, segs, owner);
             if (demig_smem_bytes(G, widest, p->M) + static_reserve <= (size_t)smem_optin) break;
@@ -1419,15 +1470,16 @@ static int demig_prepare(img2d_plan *p, int slab)
         fn = find_demig(G, p->L);
         smem = demig_smem_bytes(G, widest, p->M);
     }
-    if (!fn) return fail(IMG2D_EINVAL, "no demigration kernel for this configuration");
-    IMG2D_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (!fn && !rows_fn) return fail(IMG2D_EINVAL, "no demigration kernel for this configuration");
+    const void *any_fn = rows_fn ? (const void *)rows_fn : (const void *)fn;
+    IMG2D_CUDA(cudaFuncSetAttribute(any_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     std::vector<int2> items;
     std::vector<int> gorder(groups.size());
     std::iota(gorder.begin(), gorder.end(), 0);
     std::stable_sort(gorder.begin(), gorder.end(), [&](int a, int b) { return groups[a].W > groups[b].W; });
     for (int g : gorder)
         for (int j = 0; j < p->nf; ++j) items.push_back(make_int2(g, j));
-    int grid = 0;
+    int grid = 0, block = kAdjWarps * 32;
     long long work_cta = 0;   // float2 elements of per-CTA work area
     long long cache_item = 0; // float2 elements of kept checkpoints per item
     if (K) {
@@ -1449,6 +1501,32 @@ static int demig_prepare(img2d_plan *p, int slab)
         const long long pe4 = (long long)kDcPC * kDcQ;  // float4 per plane
         work_cta = 2 * (long long)(nslab + slab + 1) * pe4;
         cache_item = 2 * (long long)K * nslab * pe4;
+    } else if (rows_fn) {
+        // warps: a forward step takes a round per 32 positions and warp, a transposed one (2.4 times
+        // as long) per 64; the more warps share an SM the longer a round (rows_launch)
+        int smem_sm = 0;
+        IMG2D_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+        const int wp = rows_adj_wp(widest), n64 = wp / kRowsAdjPos;
+        const long long n_items = (long long)items.size();
+        double best = 1e30;
+        for (int w = 1; w <= std::min(n64, kRowsThreads / 32); ++w) {
+            const long long c = std::min<long long>(16 / w, smem_sm / (long long)(smem + 1024));
+            if (c < 1) continue;
+            const double rounds = (2 * n64 + w - 1) / w + 2.4 * ((n64 + w - 1) / w);
+            auto wave = [&](long long per_sm) { return rounds * (1.0 + per_sm * w / 6.0); };
+            const long long full = n_items / (nsm * c), rest = n_items % (nsm * c);
+            const double t = full * wave(c) + (rest ? wave((rest + nsm - 1) / nsm) : 0.0);
+            if (t < best) {
+                best = t;
+                block = 32 * w;
+            }
+        }
+        int bps = 0;
+        IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, any_fn, block, smem));
+        if (bps <= 0) return fail(IMG2D_ECUDA, "the row-split demigration kernel does not fit on an SM");
+        grid = (int)std::min<size_t>(items.size(), (size_t)nsm * bps);
+        work_cta = (long long)p->nextrap * wp * G;
+        cache_item = work_cta;
     } else {
         int bps = 0;
         IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kAdjWarps * 32, smem));
@@ -1463,7 +1541,7 @@ static int demig_prepare(img2d_plan *p, int slab)
     if ((rc = p->adj_segs.ensure(segs.size() * sizeof(int4)))) return rc;
     if ((rc = p->adj_owner.ensure(owner.size() * sizeof(int16_t)))) return rc;
     if ((rc = p->adj_counter.ensure(sizeof(int)))) return rc;
-    if ((rc = p->adj_work.ensure((size_t)grid * work_cta * sizeof(float2)))) return rc;
+    if (!rows_fn && (rc = p->adj_work.ensure((size_t)grid * work_cta * sizeof(float2)))) return rc;
     IMG2D_CUDA(cudaMemcpy(p->adj_items.p, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice));
     IMG2D_CUDA(cudaMemcpy(p->adj_groups.p, groups.data(), groups.size() * sizeof(GroupDesc), cudaMemcpyHostToDevice));
     IMG2D_CUDA(cudaMemcpy(p->adj_segs.p, segs.data(), segs.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -1472,7 +1550,10 @@ static int demig_prepare(img2d_plan *p, int slab)
     p->adj_grid = grid;
     p->adj_items_n = (int)items.size();
     p->adj_wmax = widest;
-    p->adj_block = K ? kDcNW * 32 : kAdjWarps * 32;
+    p->adj_block = K ? kDcNW * 32 : block;
+    p->adj_rows = rows_fn != nullptr;
+    p->adj_rows_fn = rows_fn;
+    p->adj_full_cache = rows_fn && (long long)items.size() * cache_item <= kDemigRowsCacheElems;
     p->adj_cluster = K;
     p->adj_work_cta = work_cta;
     p->adj_cache_item = cache_item;
@@ -1824,8 +1905,25 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
     if (source_mode == IMG2D_SOURCE_REUSE && !p->adj_cache_valid)
         return fail(IMG2D_EINVAL, "no kept source checkpoints on this plan (call with IMG2D_SOURCE_KEEP first, "
                                   "after the last set_model, with the same slab depth)");
+    if (p->adj_rows) {
+        rc = IMG2D_OK;
+        if (source_mode == IMG2D_SOURCE_KEEP)
+            rc = p->adj_cache.ensure(p->adj_full_cache ? (size_t)p->adj_items_n * p->adj_cache_item * sizeof(float2) : 16);
+        if (!rc && !(p->adj_full_cache && source_mode != IMG2D_SOURCE_RECOMPUTE))
+            rc = p->adj_work.ensure((size_t)p->adj_grid * p->adj_work_cta * sizeof(float2));
+        if (rc == IMG2D_ENOMEM && source_mode != IMG2D_SOURCE_REUSE) {
+            // too little memory for every S_l: the slab kernel
+            p->adj_cache.release();
+            p->adj_work.release();
+            p->adj_allow_rows = p->adj_rows = false;
+            p->adj_rows_fn = nullptr;
+            p->adj_slab = 0;
+            rc = demig_prepare(p, slab_depth);
+        }
+        if (rc) return rc;
+    }
     const long long cache_elems = (long long)p->adj_items_n * p->adj_cache_item;  // float2
-    if (source_mode == IMG2D_SOURCE_KEEP) {
+    if (source_mode == IMG2D_SOURCE_KEEP && !p->adj_rows) {
         if ((rc = p->adj_cache.ensure((size_t)cache_elems * sizeof(float2)))) return rc;
     }
     cudaStream_t st = (cudaStream_t)stream;
@@ -1875,6 +1973,18 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_fn, a));
+    } else if (p->adj_rows) {
+        if (!p->rows_tab_set && (rc = set_rows_table(p, st))) return rc;
+        RowsAdjArgs ra{};
+        ra.d = a;
+        if (!p->adj_full_cache) ra.d.ckpt_mode = IMG2D_SOURCE_RECOMPUTE;
+        ra.tab_rows = p->tab_rows.p;
+        const RowsStarts rs = rows_starts(p->L);
+        for (int i = 0; i < 4; ++i) ra.row_start[i] = rs.s[i];
+        ra.row_apart = rs.apart;
+        ra.planes = ra.d.ckpt_mode ? p->adj_cache.p : p->adj_work.p;
+        ra.plane = rows_adj_wp(p->adj_wmax);
+        p->adj_rows_fn<<<p->adj_grid, p->adj_block, p->adj_smem, st>>>(ra);
     } else {
         p->adj_fn<<<p->adj_grid, p->adj_block, p->adj_smem, st>>>(a);
     }
@@ -1890,12 +2000,12 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
 int img2d_plan_describe_demigration(const img2d_plan *p, char *buf, int buflen)
 {
     if (!p || !buf || buflen <= 0) return fail(IMG2D_EINVAL, "bad describe arguments");
-    if (!p->adj_fn) return fail(IMG2D_EINVAL, "no demigration has run on this plan yet");
+    if (!p->adj_fn && !p->adj_rows_fn) return fail(IMG2D_EINVAL, "no demigration has run on this plan yet");
     snprintf(buf, buflen,
              "{\"kernel\": \"%s\", \"cluster\": %d, \"G\": %d, \"X\": 8, \"L\": %d, \"grid\": %d, \"block\": %d, "
              "\"smem\": %zu, \"items\": %d, \"max_union_width\": %d, \"slab\": %d, \"slabs\": %d, "
              "\"workspace_bytes\": %zu, \"source_cache_bytes\": %zu, \"ring\": %s}",
-             p->adj_cluster ? "demigrate_cluster" : "demigrate", p->adj_cluster, p->adj_G, p->L, p->adj_grid,
+             p->adj_rows ? "demigrate_rows" : (p->adj_cluster ? "demigrate_cluster" : "demigrate"), p->adj_cluster, p->adj_G, p->L, p->adj_grid,
              p->adj_block, p->adj_smem, p->adj_items_n, p->adj_wmax, p->adj_slab,
              p->adj_nslab, p->adj_work.bytes, p->adj_cache.bytes, p->adj_ring ? "true" : "false");
     return IMG2D_OK;

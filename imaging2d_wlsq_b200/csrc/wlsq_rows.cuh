@@ -19,8 +19,8 @@
 // Wavefields of an item (G slots x one frequency) stay in shared memory, two buffers in turn, one
 // barrier per depth step.  A position is one float4 (S.re, S.im, R.re, R.im), R conjugated in the
 // single-table mode; one unused float4 after every 8 positions spreads a quad's four tap ranges over
-// the banks.  The operator row offsets of the next step are loaded at the start of a step and stored
-// to shared memory at its end.
+// the banks.  The operator row offsets come from shared memory, where each step stores those of the
+// step after next.
 //
 // Image: the first item of a CTA stores its rows of the CTA's partial image (nothing has to be zeroed
 // or read), later ones add with Kahan compensation; the reduction reads what the CTA's item count
@@ -106,8 +106,8 @@ __host__ __device__ inline size_t rows_smem_bytes(int G, int W, int L)
 // three or four lanes overlap, each holds a half, a quarter (the first of three a half) or a quarter
 // of the tap: the products then add up to the tap's (scaling by a power of two is exact) and
 // infinities and NaN come out as from the whole tap.
-__global__ void rows_table_kernel(const cpx *__restrict__ tabF, const cpx *__restrict__ tabB, int L, int NP, RowsStarts st,
-                                  int nk, float *__restrict__ out)
+__global__ void rows_table_kernel(const cpx *__restrict__ tabF, const cpx *__restrict__ tabB, int stride, int L,
+                                  int NP, RowsStarts st, int nk, float *__restrict__ out)
 {
     const int nt = tabB ? 2 : 1;
     const int per_row = 8 * NP * nt;  // complex elements
@@ -128,7 +128,7 @@ __global__ void rows_table_kernel(const cpx *__restrict__ tabF, const cpx *__res
             }
         }
         const float w = m == 1 ? 1.f : (m == 2 || (m == 3 && before == 0) ? 0.5f : 0.25f);
-        const cpx v = k < L ? (which ? tabB : tabF)[(long long)row * L + k] : cpx{0.f, 0.f};
+        const cpx v = k < L ? (which ? tabB : tabF)[(long long)row * stride + k] : cpx{0.f, 0.f};
         out[2 * e] = w * v.re;
         out[2 * e + 1] = w * v.im;
     }

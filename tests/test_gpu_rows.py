@@ -5,7 +5,7 @@ chunked host entry, and non-finite inputs against the general kernel."""
 import numpy as np
 import pytest
 
-from imaging2d_wlsq_b200 import migration, operators, synthetic
+from imaging2d_wlsq_b200 import lsm, migration, operators, synthetic
 from oracle import oracle
 from tests.conftest import rel_l2
 
@@ -108,3 +108,41 @@ def test_rows_non_finite_inputs_reach_what_they_reach_in_the_general_kernel(taps
         np.testing.assert_array_equal(np.isfinite(a), np.isfinite(b))
         np.testing.assert_array_equal(np.isnan(a.real), np.isnan(b.real))
         np.testing.assert_array_equal(np.isnan(a.imag), np.isnan(b.imag))
+
+
+@pytest.mark.parametrize("taps", [3, 5, 7, 9, 15, 17, 25, 31, 41, 57, 63, 65, 79])
+@pytest.mark.parametrize("ns,nx", [(1, 33), (2, 130), (3, 65), (2, 1000)])
+def test_rows_demigration_matches_oracle(taps, ns, nx):
+    """Row-split demigration, one and two slots per item (1000 positions with long operators leave
+    room for one), every source mode."""
+    import torch
+    w = _survey(ns, nx, 4, 3, taps)
+    m = np.random.default_rng(2).standard_normal((w.nextrap, w.nx)).astype(np.float32)
+    ref = oracle.demigrate_workload_f64(w, m.astype(np.float64))
+    op = lsm.MigrationOperator.for_workload(w)
+    out = []
+    for mode in ("recompute", "keep", "reuse"):
+        d = op.zeros_data()
+        op.plan.demigrate(torch.from_numpy(m).cuda(), op.wave, d, source=mode)
+        out.append(d.cpu().numpy())
+        assert rel_l2(out[-1], ref) <= 1e-5
+    assert op.plan.describe_demigration()["kernel"] == "demigrate_rows"
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    op.plan.close()
+
+
+def test_rows_demigration_with_little_memory_takes_the_slab_kernel():
+    import torch
+    from imaging2d_wlsq_b200._lib import lib
+    w = _survey(2, 256, 64, 8, 31)
+    m = np.random.default_rng(2).standard_normal((w.nextrap, w.nx)).astype(np.float32)
+    ref = oracle.demigrate_workload_f64(w, m.astype(np.float64))
+    op = lsm.MigrationOperator.for_workload(w)
+    lib().img2d_set_alloc_limit(1 << 20)  # every S_l: 8 CTAs x 64 planes of 4 KB; checkpoints: a quarter
+    try:
+        d = op.demigrate(torch.from_numpy(m).cuda())
+    finally:
+        lib().img2d_set_alloc_limit(0)
+    assert op.plan.describe_demigration()["kernel"] == "demigrate"
+    assert rel_l2(d.cpu().numpy(), ref) <= 1e-5
+    op.plan.close()
