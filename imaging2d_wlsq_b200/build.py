@@ -7,6 +7,7 @@ Outputs (git-ignored, shipped with the tree):
   oracle/_ref/extrapolation_cpu.so                   the reference's own CPU library (when its
                                                      sources are present on this machine)
 """
+import glob
 import os
 import subprocess
 import sys
@@ -19,7 +20,7 @@ REFERENCE_TREE = "/root/reference"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 LIB = os.path.join(PKG, "libimaging2d_wlsq_b200.so")
 SOURCES = [os.path.join(PKG, "csrc", "wlsq_capi.cu")]
-HEADERS = [os.path.join(PKG, "csrc", "wlsq_kernels.cuh"), os.path.join(ROOT, "include", "imaging2d_wlsq_b200.h")]
+HEADERS = sorted(glob.glob(os.path.join(PKG, "csrc", "*.cuh"))) + [os.path.join(ROOT, "include", "imaging2d_wlsq_b200.h")]
 DROPINS = {
     "extrapolation_cpu.so": ["-DIMG2D_DROPIN_HOST"],
     "extrapolation_gpu.so": ["-DIMG2D_DROPIN_DEVICE=0"],

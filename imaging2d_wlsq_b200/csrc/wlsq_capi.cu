@@ -2188,16 +2188,15 @@ int img2d_ricker_sources(int ns, int nt, int nx, double dt, double x_first, doub
     return IMG2D_OK;
 }
 
-int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const float *d_records,
-                             const int *shot_x0, const int *shot_nx, img2d_c64 *d_out, void *stream)
+// Apertures of a front-end call: per-shot start, width and offset of the packed block.
+static int spectra_layout(int ns, int nt, int nx, int nf, int nt_rows, const int *shot_x0, const int *shot_nx,
+                          std::vector<int> &x0, std::vector<int> &w, std::vector<long long> &off)
 {
-    int rc;
-    if ((rc = check_device())) return rc;
     if (ns <= 0 || nt <= 0 || nx <= 0 || nf <= 0 || nf > nt || nt_rows < nf)
         return fail(IMG2D_EINVAL, "invalid dimensions (need ns, nt, nx > 0, 0 < nf <= nt, nt_rows >= nf)");
-    if (!d_records || !d_out) return fail(IMG2D_EINVAL, "null pointer argument");
-    std::vector<int> x0(ns, 0), w(ns, nx);
-    std::vector<long long> off(ns, 0);
+    x0.assign(ns, 0);
+    w.assign(ns, nx);
+    off.assign(ns, 0);
     long long acc = 0;
     for (int s = 0; s < ns; ++s) {
         if (shot_x0) x0[s] = shot_x0[s];
@@ -2207,21 +2206,78 @@ int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const 
         off[s] = acc;
         acc += (long long)nt_rows * w[s];
     }
-    cudaStream_t st = (cudaStream_t)stream;
+    return IMG2D_OK;
+}
+
+// Front-end scratch of one device (transform tables, cuFFT spectra), kept and grown on demand.  A
+// call holds the lock until its work has finished, so that the scratch has one user.
+struct FrontScratch {
+    DevBuf tables, spec;
+    std::map<std::vector<long long>, cufftHandle> plans;  // by (nt, nx)
+};
+static std::mutex g_front_mu;
+static std::map<int, FrontScratch> g_front;
+
+// The two-stage transform of records of nt samples: the divisor N1 <= 31 with the fewest
+// multiply-adds per trace; none (N1 = 0) where that exceeds 150 nt (a prime nt: cuFFT is taken) or the
+// inner sums of 8 traces do not fit in shared memory.  16 traces per CTA (64-byte reads) unless only 8
+// leave room for two CTAs per SM.
+static SpecPlan spec_plan(int nt, int nf, size_t smem_optin)
+{
+    SpecPlan best{};
+    double best_cost = 150.0 * nt;
+    for (int N1 = 1; N1 <= 31 && N1 <= nt; ++N1) {
+        if (nt % N1) continue;
+      for (int M : {8, 10}) {
+        SpecPlan p{};
+        p.M = M;
+        p.N1 = N1;
+        p.N2 = nt / N1;
+        p.K1 = N1 / 2 + 1;
+        p.mp = ((nf + N1 - 1) / N1 + M - 1) / M * M;
+        const size_t per = (size_t)p.N2 * p.K1 * sizeof(float2), table = (size_t)p.N2 * p.mp * sizeof(float2);
+        p.bs = table <= 8192;
+        const size_t more = p.bs ? table : 0, room = smem_optin - 6144;
+        p.C = 16 * per + more <= room / 2 ? 16 : (8 * per + more <= room / 2 ? 8 : (16 * per + more <= room ? 16 : 8));
+        p.smem = per * p.C + more;
+        if (p.smem > room) continue;
+        double cost = 2.0 * ((p.K1 + kSpecKC - 1) / kSpecKC * kSpecKC) * p.N2 * (N1 / 2);
+        for (int k1 = 0; k1 < std::min(N1, nf); ++k1) cost += 4.0 * p.N2 * ((nf - 1 - k1) / (N1 * M) + 1) * M;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = p;
+        }
+      }
+    }
+    return best;
+}
+
+static SpecShots spec_shots(int s0, int n, const std::vector<int> &x0, const std::vector<int> &w,
+                            const std::vector<long long> &off)
+{
+    SpecShots sh{};
+    for (int i = 0; i < n; ++i) {
+        sh.x0[i] = x0[s0 + i];
+        sh.w[i] = w[s0 + i];
+        sh.off[i] = off[s0 + i];
+    }
+    return sh;
+}
+
+// cuFFT path: the real-to-complex transforms along time of groups of shots, then the packing kernel.
+static int spectra_by_cufft(FrontScratch &fs, int ns, int nt, int nx, int nf, const float *d_records,
+                            const std::vector<int> &x0, const std::vector<int> &w, const std::vector<long long> &off,
+                            cpx *d_out, cudaStream_t st)
+{
+    int rc;
     // shots per transform group: their spectra (nt/2+1 rows) in at most 512 MB of scratch
     const long long shot_spec = (long long)(nt / 2 + 1) * nx;
     const int group = (int)std::max<long long>(1, std::min<long long>(ns, (512ll << 20) / (shot_spec * 8)));
-    int dev = 0;
-    IMG2D_CUDA(cudaGetDevice(&dev));
-    // One plan per (device, nt, nx), kept for the process: the nx transforms of length nt of one
-    // shot, element (t, x) at x + t*nx in and at x + j*nx out; shots are issued one by one.  The
-    // plans are shared, so the lock is held while this call issues its transforms.
-    static std::mutex plan_mu;
-    static std::map<std::vector<long long>, cufftHandle> plans;
-    std::lock_guard<std::mutex> plan_lock(plan_mu);
-    const std::vector<long long> key = {dev, nt, nx};
-    auto itp = plans.find(key);
-    if (itp == plans.end()) {
+    // One plan per (nt, nx), kept for the process: the nx transforms of length nt of one shot,
+    // element (t, x) at x + t*nx in and at x + j*nx out; shots are issued one by one.
+    const std::vector<long long> key = {nt, nx};
+    auto itp = fs.plans.find(key);
+    if (itp == fs.plans.end()) {
         int n[1] = {nt};
         int inembed[1] = {nt}, onembed[1] = {nt / 2 + 1};
         cufftHandle h;
@@ -2231,15 +2287,15 @@ int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const 
             cufftDestroy(h);
             return fail(IMG2D_ECUDA, "cufftMakePlanMany (real-to-complex along time) failed");
         }
-        itp = plans.emplace(key, h).first;
+        itp = fs.plans.emplace(key, h).first;
     }
     const cufftHandle plan = itp->second;
     if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return fail(IMG2D_ECUDA, "cufftSetStream failed");
-    // the spectra scratch (up to 512 MB) is kept per device with the plans, grown on demand
-    static std::map<int, DevBuf> spec_scratch;
-    DevBuf &spec = spec_scratch[dev];
-    if ((rc = spec.ensure((size_t)group * shot_spec * sizeof(cpx)))) return rc;
-    cpx *d_spec = spec.as<cpx>();
+    // cuFFT reads 8-byte pairs: with an odd nt * nx every other shot goes through an aligned copy
+    const bool odd = ns > 1 && ((long long)nt * nx & 1);
+    if ((rc = fs.spec.ensure((size_t)group * shot_spec * sizeof(cpx) + (odd ? (size_t)nt * nx * sizeof(float) : 0)))) return rc;
+    cpx *d_spec = fs.spec.as<cpx>();
+    float *aligned = reinterpret_cast<float *>(d_spec + (long long)group * shot_spec);
     Scratch sc;
     int *d_x0, *d_w;
     long long *d_off;
@@ -2253,15 +2309,104 @@ int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const 
         const int nsc = std::min(group, ns - s0);
         for (int k = 0; k < nsc; ++k) {
             cufftReal *in = const_cast<cufftReal *>(d_records + (long long)(s0 + k) * nt * nx);
+            if (odd && ((s0 + k) & 1)) {
+                IMG2D_CUDA(cudaMemcpyAsync(aligned, in, (size_t)nt * nx * sizeof(float), cudaMemcpyDeviceToDevice, st));
+                in = aligned;
+            }
             cufftComplex *o = reinterpret_cast<cufftComplex *>(d_spec + (long long)k * shot_spec);
             if (cufftExecR2C(plan, in, o) != CUFFT_SUCCESS) return fail(IMG2D_ECUDA, "cufftExecR2C failed");
         }
         const long long total = (long long)nsc * nf * nx;
         const int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 32);
-        pack_spectra_kernel<<<blocks, 256, 0, st>>>(s0, nsc, nt, nx, nf, d_spec, d_x0, d_w, d_off, (cpx *)d_out);
+        pack_spectra_kernel<<<blocks, 256, 0, st>>>(s0, nsc, nt, nx, nf, d_spec, d_x0, d_w, d_off, d_out);
         IMG2D_CUDA(cudaGetLastError());
     }
     IMG2D_CUDA(cudaStreamSynchronize(st));  // the descriptors are freed on return
+    return IMG2D_OK;
+}
+
+int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const float *d_records,
+                             const int *shot_x0, const int *shot_nx, img2d_c64 *d_out, void *stream)
+{
+    int rc;
+    if ((rc = check_device())) return rc;
+    std::vector<int> x0, w;
+    std::vector<long long> off;
+    if ((rc = spectra_layout(ns, nt, nx, nf, nt_rows, shot_x0, shot_nx, x0, w, off))) return rc;
+    if (!d_records || !d_out) return fail(IMG2D_EINVAL, "null pointer argument");
+    cudaStream_t st = (cudaStream_t)stream;
+    int dev = 0, smem_optin = 0;
+    IMG2D_CUDA(cudaGetDevice(&dev));
+    IMG2D_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    std::lock_guard<std::mutex> lock(g_front_mu);
+    FrontScratch &fs = g_front[dev];
+    const SpecPlan pl = spec_plan(nt, nf, (size_t)smem_optin);
+    if (!pl.N1) return spectra_by_cufft(fs, ns, nt, nx, nf, d_records, x0, w, off, (cpx *)d_out, st);
+    const size_t n1 = (size_t)kSpecK * kSpecK, n2 = (size_t)pl.N2 * pl.mp, n3 = (size_t)nt;
+    if ((rc = fs.tables.ensure((n1 + n2 + n3) * sizeof(float2)))) return rc;
+    float2 *T1 = fs.tables.as<float2>(), *B = T1 + n1, *A = B + n2;
+    spec_tables_kernel<<<(int)std::min<size_t>((n1 + n2 + n3 + 255) / 256, 148 * 4), 256, 0, st>>>(pl, nt, T1, B, A);
+    IMG2D_CUDA(cudaGetLastError());
+#define IMG2D_SPEC(C, M) (pl.bs ? record_spectra_kernel<C, M, true> : record_spectra_kernel<C, M, false>)
+    auto kernel = pl.C == 16 ? (pl.M == 8 ? IMG2D_SPEC(16, 8) : IMG2D_SPEC(16, 10))
+                             : (pl.M == 8 ? IMG2D_SPEC(8, 8) : IMG2D_SPEC(8, 10));
+#undef IMG2D_SPEC
+    IMG2D_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+    for (int s0 = 0; s0 < ns; s0 += kSpecShots) {
+        const int n = std::min(kSpecShots, ns - s0);
+        kernel<<<dim3((nx + pl.C - 1) / pl.C, n), 256, pl.smem, st>>>(pl, spec_shots(s0, n, x0, w, off), s0, nt, nx, nf,
+                                                                      d_records, T1, B, A, (cpx *)d_out);
+        IMG2D_CUDA(cudaGetLastError());
+    }
+    IMG2D_CUDA(cudaStreamSynchronize(st));
+    return IMG2D_OK;
+}
+
+int img2d_source_spectra(int ns, int nt, int nx, int nf, int nt_rows, double dt, double x_first, double dx,
+                         double depth_offset, double v, double fpeak, const double *src_x, const int *shot_x0,
+                         const int *shot_nx, img2d_c64 *d_out, void *stream)
+{
+    int rc;
+    if ((rc = check_device())) return rc;
+    if (!(dt > 0.0) || !(dx > 0.0) || !(v > 0.0))
+        return fail(IMG2D_EINVAL, "invalid source-wavelet dimensions or spacing");
+    std::vector<int> x0, w;
+    std::vector<long long> off;
+    if ((rc = spectra_layout(ns, nt, nx, nf, nt_rows, shot_x0, shot_nx, x0, w, off))) return rc;
+    if (!src_x || !d_out) return fail(IMG2D_EINVAL, "null pointer argument");
+    cudaStream_t st = (cudaStream_t)stream;
+    // half width of the samples that are not zero in float32: (pi fpeak t)^2 = 150
+    const double tw = std::sqrt(150.0) / (3.141592653589793 * std::fabs(fpeak));
+    const double span = 2.0 * tw / dt + 3.0;
+    if (span > 384.0 || !(span > 0.0)) {
+        // a wavelet of more samples (or a constant): through the time domain
+        float *d_t = nullptr;
+        Scratch sc;
+        if ((rc = sc.alloc(&d_t, (size_t)ns * nt * nx * sizeof(float)))) return rc;
+        if ((rc = img2d_ricker_sources(ns, nt, nx, dt, x_first, dx, depth_offset, v, fpeak, src_x, d_t, stream))) return rc;
+        return img2d_records_to_spectra(ns, nt, nx, nf, nt_rows, d_t, shot_x0, shot_nx, d_out, stream);
+    }
+    const int nsup = std::min(nt, (int)span), kp = (nf + kSrcK - 1) / kSrcK * kSrcK;
+    int dev = 0;
+    IMG2D_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_front_mu);
+    FrontScratch &fs = g_front[dev];
+    const size_t nw = ((size_t)nt + 1) / 2 * 2, nu = (size_t)nsup * kp;
+    if ((rc = fs.tables.ensure((nw + nu) * sizeof(float2)))) return rc;
+    float2 *W = fs.tables.as<float2>(), *U = W + nw;
+    source_tables_kernel<<<(int)std::min<size_t>((nw + nu + 255) / 256, 148 * 4), 256, 0, st>>>(nt, (int)nw, nsup, kp, W, U);
+    IMG2D_CUDA(cudaGetLastError());
+    const size_t smem = (size_t)nsup * kSrcCols * sizeof(float);
+    IMG2D_CUDA(cudaFuncSetAttribute(source_spectra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int s0 = 0; s0 < ns; s0 += kSpecShots) {
+        const int n = std::min(kSpecShots, ns - s0);
+        SpecShots sh = spec_shots(s0, n, x0, w, off);
+        for (int i = 0; i < n; ++i) sh.sx[i] = src_x[s0 + i];
+        source_spectra_kernel<<<dim3((nx + kSrcCols - 1) / kSrcCols, n, nf > 64 ? 2 : 1), 256, smem, st>>>(sh, nt, nx, nf, nsup, kp, dt, x_first, dx,
+                                                                         depth_offset, v, fpeak, tw, W, U, (cpx *)d_out);
+        IMG2D_CUDA(cudaGetLastError());
+    }
+    IMG2D_CUDA(cudaStreamSynchronize(st));
     return IMG2D_OK;
 }
 

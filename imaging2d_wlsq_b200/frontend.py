@@ -8,7 +8,7 @@ Mirrors the per-shot preparation of the reference driver (main.py:105-123):
     pulse_back_fs[s] = scipy.fftpack.fft(pulse_back_st[s], axis=0)
 
 with tj = j*dt, xi = xmin + (i+1)*dx and v = velocity[0, 0] (main.py:111-113).  The wavelet and the
-transform run as CUDA kernels (img2d_ricker_sources, img2d_records_to_spectra); only the first nf
+transform run as CUDA kernels (img2d_source_spectra, img2d_records_to_spectra); only the first nf
 frequency rows, the ones the extrapolation uses, are computed, straight into the packed per-shot
 aperture layout of migration.Plan.
 """
@@ -47,7 +47,9 @@ def records_to_spectra(records, nf, nt_rows=None, shot_x0=None, shot_nx=None, ou
     widths = np.full(ns, nx, dtype=np.int64) if wn is None else wn.astype(np.int64)
     total = int(nt_rows * widths.sum())
     if out is None:
-        out = torch.zeros(total, dtype=torch.complex64, device=records.device)
+        # rows beyond nf are zero
+        new = torch.zeros if nt_rows > nf else torch.empty
+        out = new(total, dtype=torch.complex64, device=records.device)
     elif out.numel() < total or out.dtype != torch.complex64:
         raise ValueError("out is too small or not complex64")
     check(lib().img2d_records_to_spectra(ns, nt, nx, int(nf), int(nt_rows), ptr(records),
@@ -57,14 +59,29 @@ def records_to_spectra(records, nf, nt_rows=None, shot_x0=None, shot_nx=None, ou
     return out
 
 
+def source_spectra(ns, nt, nx, nf, dt, x_first, dx, depth_offset, v, src_x, fpeak=30.0, nt_rows=None, device=None):
+    """records_to_spectra of ricker_sources' wavelets (full aperture), without the time-domain array."""
+    import torch
+    dev = device or torch.device("cuda")
+    nt_rows = nt_rows or nf
+    sx = np.ascontiguousarray(src_x, dtype=np.float64)
+    if sx.shape != (ns,):
+        raise ValueError("src_x must have one position per source")
+    new = torch.zeros if nt_rows > nf else torch.empty  # rows beyond nf are zero
+    out = new(int(ns * nt_rows * nx), dtype=torch.complex64, device=dev)
+    check(lib().img2d_source_spectra(ns, nt, nx, int(nf), int(nt_rows), float(dt), float(x_first), float(dx),
+                                     float(depth_offset), float(v), float(fpeak), sx.ctypes.data, None, None, ptr(out),
+                                     ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
+    return out
+
+
 def prepare_shots(records, shot_isx, nf, xmin, dx, dt, zinit, dz, v, fpeak=30.0, nt_rows=None):
     """Source and receiver spectra of main.py:105-123 for device records (ns, nt, nx) float32 and
     the shots' source indices.  Returns (wave, shot): packed complex64 device vectors with
     nt_rows (default nf) rows per shot, full aperture, ready for migration.Plan.execute."""
     ns, nt, nx = records.shape
     sx = xmin + np.asarray(shot_isx, dtype=np.float64) * dx
-    src_t = ricker_sources(ns, nt, nx, dt, xmin + dx, dx, dz - zinit, v, sx, fpeak=fpeak, device=records.device)
-    wave = records_to_spectra(src_t, nf, nt_rows=nt_rows)
-    del src_t
+    wave = source_spectra(ns, nt, nx, nf, dt, xmin + dx, dx, dz - zinit, v, sx, fpeak=fpeak, nt_rows=nt_rows,
+                          device=records.device)
     shot = records_to_spectra(records, nf, nt_rows=nt_rows)
     return wave, shot

@@ -197,13 +197,19 @@ int img2d_measure_l2_bandwidth(double *gbs);
  * records or the wavelets above) -> d_out packed like the migration's wave/shot buffers (per shot
  * nt_rows rows of that shot's aperture [shot_x0[s], shot_x0[s] + shot_nx[s]), NULL = full
  * aperture), rows j < nf set to sum_t rec[t][x] exp(-2 pi i j t / nt), other rows untouched.  The
- * transform is a single-precision real-to-complex cuFFT along time (as the reference's transform of
- * float32 records is single precision), rows above nt/2 by conjugate symmetry.  shot_x0 / shot_nx
+ * transform is single precision, as the reference's transform of float32 records is: two stages of
+ * nt = N1 N2 in shared memory, or a real-to-complex cuFFT for lengths without a suitable divisor.  shot_x0 / shot_nx
  * are host arrays; the call returns when d_out is written.
  * ---------------------------------------------------------------------------------------- */
 int img2d_ricker_sources(int ns, int nt, int nx, double dt, double x_first, double dx,
                          double depth_offset, double v, double fpeak, const double *src_x,
                          float *d_out, void *stream);
+/* img2d_source_spectra: the first nf rows of img2d_records_to_spectra of img2d_ricker_sources' wavelets,
+ * without forming them in the time domain (samples that are zero in float32 are left out of the sum).
+ * src_x, shot_x0 and shot_nx are host arrays; the call returns when d_out is written. */
+int img2d_source_spectra(int ns, int nt, int nx, int nf, int nt_rows, double dt, double x_first, double dx,
+                         double depth_offset, double v, double fpeak, const double *src_x, const int *shot_x0,
+                         const int *shot_nx, img2d_c64 *d_out, void *stream);
 int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const float *d_records,
                              const int *shot_x0, const int *shot_nx, img2d_c64 *d_out, void *stream);
 
