@@ -1060,7 +1060,30 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             }
         }
     }
+    // The 16-slot default: the wide kernel's step with 8 lanes per group (16 slots x 512 positions per
+    // CTA, clusters as cluster2's), reported as the cluster2 variant after those of the table.
+    auto try_wide16 = [&]() {
+        const bool stage = wide_stage_smem_bytes<Wide16Shape>(M) + static_reserve <= (size_t)smem_optin;
+        const size_t smemw = stage ? wide_stage_smem_bytes<Wide16Shape>(M) : wide_smem_bytes<Wide16Shape>(M);
+        if (smemw + static_reserve > (size_t)smem_optin) return false;
+        KernelFn wf = stage ? migrate_wide_kernel<1, true, false, 8> : migrate_wide_kernel<1, false, false, 8>;
+        const int widest = make_groups(Wide16Shape::G);
+        const int K = (widest + Wide16Shape::PC - 1) / Wide16Shape::PC;
+        if (!(K <= 8 || (K <= kMaxCluster && clusters_that_fit((const void *)wf, K, Wide16Shape::NW * 32, smemw) > 0)))
+            return false;
+        p->cluster = K;
+        p->G = Wide16Shape::G;
+        p->fixed = true;
+        p->fn = wf;
+        p->smem = smemw;
+        p->max_w = widest;
+        p->block = Wide16Shape::NW * 32;
+        p->variant = kNumCluster2 + (stage ? 0 : 1);
+        p->kname = "migrate_cluster2";
+        return true;
+    };
     if (!p->rows && want_wide) try_wide();
+    if (!p->cluster && !p->rows && cluster_ok && !explicit_kernel && p->L >= 7) try_wide16();
     if (!p->cluster && !p->rows && cluster_ok && !(flags & (IMG2D_FLAG_CLUSTER_V1 | wide_flags)) &&
         p->L >= 7) {
         // the default ring variant needs 33 KB more shared memory than the staged one: long

@@ -42,8 +42,9 @@
 
 namespace img2d {
 
-struct WideShape {
-    static constexpr int Q = 4;            // lanes per position group
+template <int LANES>
+struct WideShapeQ {
+    static constexpr int Q = LANES;        // lanes per position group
     static constexpr int G = 2 * Q;        // lane slots per item (two per lane)
     static constexpr int P = 32 / Q;       // position groups per warp
     static constexpr int NW = 16;          // warps per CTA
@@ -52,24 +53,28 @@ struct WideShape {
     static constexpr int NG = NW * P;      // lane groups per CTA (128)
     static constexpr int RING = 8 * kRingSlots + 1;  // float4 per lane group's ring (+1 pad)
 };
+typedef WideShapeQ<4> WideShape;
+typedef WideShapeQ<8> Wide16Shape;
 
 // Shared memory: ext[PC + 2 MP] rows + staging[2 parity][2 side][MP] rows (8 float4 per row) +
 // the operator-pair rings.
+template <class S = WideShape>
 __host__ __device__ inline size_t wide_smem_bytes(int M)
 {
     const int mp = cluster2_mp(M);
-    return (size_t)((WideShape::PC + 2 * mp) + 4 * mp) * WideShape::G * 16 +
-           (size_t)WideShape::NG * WideShape::RING * 16;
+    return (size_t)((S::PC + 2 * mp) + 4 * mp) * S::G * 16 + (size_t)S::NG * S::RING * 16;
 }
 
 // Step-ahead stage (STAGE): per thread 6 words after the rings, the aligned index words holding the
 // next depth step's operator indices of its two outputs and this step's Kahan partial and
 // compensation values of its two positions.  Each thread reads only its own words, then refills
 // them with cp.async for a later step.
-constexpr int kWideStageWords = 6;
+template <class S = WideShape>
+__host__ __device__ constexpr int wide_stage_words() { return 3 * (S::X / S::Q); }
+template <class S = WideShape>
 __host__ __device__ inline size_t wide_stage_smem_bytes(int M)
 {
-    return wide_smem_bytes(M) + (size_t)WideShape::NW * 32 * kWideStageWords * 4;
+    return wide_smem_bytes<S>(M) + (size_t)S::NW * 32 * wide_stage_words<S>() * 4;
 }
 
 // BULK: two transaction-count barriers per warp after the stage words (or the rings), one per
@@ -128,7 +133,11 @@ __device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, unsign
 }
 
 // float4 column of half h (0 = S, 1 = conj R) of lane q in row pos
-__device__ __forceinline__ int wide_col(int pos, int q, int h) { return 2 * q + (h ^ ((pos >> 3) & 1)); }
+template <int Q>
+__device__ __forceinline__ int wide_col(int pos, int q, int h)
+{
+    return Q == 8 ? q + 8 * h : 2 * q + (h ^ ((pos >> 3) & 1));
+}
 
 template <int ARITH>
 __device__ __forceinline__ void wide_mac(float (&c)[8], float fr, float fi, const float4 &va, const float4 &vb)
@@ -166,11 +175,14 @@ __device__ __forceinline__ void wide_mac(float (&c)[8], float fr, float fi, cons
 // chunk completing on one of two transaction-count barriers of the warp (alternating), where the
 // cp.async ring would wait for a commit group.  A chunk is issued where the cp.async ring copies
 // its later iteration and waited for where the ring waits for its first one.
-template <int ARITH, bool STAGE, bool BULK = false>
-__global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(MigrateArgs a)
+template <int ARITH, bool STAGE, bool BULK = false, int LANES = 4>
+__global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_kernel(MigrateArgs a)
 {
-    using S = WideShape;
+    using S = WideShapeQ<LANES>;
     constexpr int Q = S::Q, G = S::G, P = S::P, X = S::X, PC = S::PC;
+    constexpr int NO = X / Q;  // outputs whose operator row, index and Kahan values a lane looks after
+    constexpr int SW = wide_stage_words<S>();
+    static_assert(!BULK || Q == 4, "the bulk-copy ring is built on 4 lanes per group");
     const int M = a.M, L = 2 * a.M + 1;
     const int MP = cluster2_mp(M);
     const int NEXT = PC + 2 * MP;
@@ -186,9 +198,9 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
     const int b = warp * P + p;  // this lane group's block: local positions [b*X, b*X+X)
     // this lane group's ring, [output][slot] float4 plus one pad, after the halo staging
     float4 *const ringb = smem + (size_t)(NEXT + 4 * MP) * G + (size_t)b * S::RING;
-    // STAGE: this thread's words [idx word of output q, of q+4, s0, c0, s1, c1]
+    // STAGE: this thread's words [index word of each of its outputs q + o Q, then s and c of each]
     unsigned *const sst = reinterpret_cast<unsigned *>(smem + (size_t)(NEXT + 4 * MP) * G + (size_t)S::NG * S::RING) +
-                          (size_t)threadIdx.x * kWideStageWords;
+                          (size_t)threadIdx.x * SW;
     const int npairs = (L + 1) >> 1;
     static_assert(X == 8 && kRingSlots == 4, "the ring schedule assumes 8 outputs per block and 4 slots");
     // BULK: this warp's two chunk barriers, the chunks it has issued and waited for (warp-uniform)
@@ -245,8 +257,8 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
             for (int x = lo + (int)threadIdx.x; x < hi; x += blockDim.x) {
                 const cpx Sv = ws[x - r0], Rv = rs[x - r0];
                 const int pos = x - c0 + MP;
-                float *fa = extf + ((size_t)pos * G + wide_col(pos, sq, 0)) * 4;
-                float *fb = extf + ((size_t)pos * G + wide_col(pos, sq, 1)) * 4;
+                float *fa = extf + ((size_t)pos * G + wide_col<Q>(pos, sq, 0)) * 4;
+                float *fb = extf + ((size_t)pos * G + wide_col<Q>(pos, sq, 1)) * 4;
                 fa[sh] = Sv.re;
                 fa[2 + sh] = Sv.im;
                 fb[sh] = Rv.re;
@@ -277,40 +289,63 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
         }
         const uint16_t *idx_j = a.idx + (long long)j * a.idx_jstride;
         const int xg = u0 + c0 + b * X;  // model position of the block's first output
-        // lane q owns outputs q and q+4 of the block: their operator rows (byte offsets into the
-        // table), next-step indices and Kahan partial-image values
-        const int xq0 = min(xg + q, a.nx - 1), xq1 = min(xg + q + Q, a.nx - 1);
-        const bool img0 = a.partial && b * X + q < own, img1 = a.partial && b * X + q + Q < own;
-        unsigned roff0 = (unsigned)idx_j[xq0] * (unsigned)row_bytes;
-        unsigned roff1 = (unsigned)idx_j[xq1] * (unsigned)row_bytes;
-        unsigned nidx01 = 0;  // next step's row indices of outputs q (low half) and q+4 (high half)
-        // STAGE: copies of the aligned index words of step ls (outputs q and q+4) and of the Kahan
-        // values of step lk (positions q and q+4) into this thread's stage words
+        // lane q owns outputs q + o Q of the block: their operator rows (byte offsets into the table),
+        // next-step indices and Kahan partial-image values
+        int xq[NO];
+        bool imgo[NO];
+        unsigned roff[NO];
+        unsigned nidx = 0;  // next step's row indices of the lane's outputs (16 bits each)
+#pragma unroll
+        for (int o = 0; o < NO; ++o) {
+            xq[o] = min(xg + q + o * Q, a.nx - 1);
+            imgo[o] = a.partial && b * X + q + o * Q < own;
+            roff[o] = (unsigned)idx_j[xq[o]] * (unsigned)row_bytes;
+        }
+        // STAGE: copies of the aligned index words of step ls and of the Kahan values of step lk into
+        // this thread's stage words
         auto stage_idx = [&](int ls) {
             const uint16_t *ip = idx_j + (long long)ls * a.idx_lstride;
-            cp_async4(sst + 0, ip + (xq0 & ~1));
-            cp_async4(sst + 1, ip + (xq1 & ~1));
+#pragma unroll
+            for (int o = 0; o < NO; ++o) cp_async4(sst + o, ip + (xq[o] & ~1));
         };
         const long long prow0 = (long long)blockIdx.x * a.nextrap * a.nx + xg + q;  // partial element of step 0
         auto stage_kahan = [&](int lk) {
             const long long e = prow0 + (long long)lk * a.nx;
-            if (img0) {
-                cp_async4(sst + 2, a.partial + e);
-                cp_async4(sst + 3, a.comp + e);
-            }
-            if (img1) {
-                cp_async4(sst + 4, a.partial + e + Q);
-                cp_async4(sst + 5, a.comp + e + Q);
+#pragma unroll
+            for (int o = 0; o < NO; ++o)
+                if (imgo[o]) {
+                    cp_async4(sst + NO + 2 * o, a.partial + e + o * Q);
+                    cp_async4(sst + NO + 2 * o + 1, a.comp + e + o * Q);
+                }
+        };
+        // Ring copies go in chunks of two iterations (v even, v and v + 1), whose pairs are 32
+        // consecutive bytes of a row: two lanes copy one output's 32 bytes, so a copy instruction of
+        // the warp touches 16 cache lines.  One lane per output and 16 bytes touched 32, and the L1 tag
+        // lookups, one line a cycle, took as long as the multiply-adds they fed (leaving the copies out
+        // altogether: 12% on the uneven survey).  rcopy[i]: the rows this lane copies from.
+        constexpr int NCP = X * 2 / Q;  // copies per lane and chunk
+        const int rh = q & 1;
+        unsigned rcopy[NCP];
+        auto spread_rows = [&]() {
+#pragma unroll
+            for (int i = 0; i < NCP; ++i) {
+                // output of copy i: (q >> 1) + i Q / 2, owned by lane (output mod Q) of the group
+                const int o = i * (Q / 2) / Q;
+                rcopy[i] = __shfl_sync(0xffffffffu, roff[o], ((q >> 1) + i * (Q / 2)) & (Q - 1), Q);
             }
         };
-        // branch-free: a pair outside the row becomes a zero-filled copy of nothing (never read)
-        auto ring_copy = [&](int u) {
+        auto ring_pair = [&](int v, bool both) {
             const char *tabb = reinterpret_cast<const char *>(a.tabF);
-            const int pr0 = u + ((X - q) >> 1), pr1 = u + ((X - q - Q) >> 1);
-            const bool ok0 = (unsigned)pr0 < (unsigned)npairs, ok1 = (unsigned)pr1 < (unsigned)npairs;
-            const int sl = u & (kRingSlots - 1);
-            cp_async16_zfill(ringb + q * kRingSlots + sl, tabb + roff0 + (ok0 ? pr0 : 0) * 16, ok0 ? 16u : 0u);
-            cp_async16_zfill(ringb + (q + Q) * kRingSlots + sl, tabb + roff1 + (ok1 ? pr1 : 0) * 16, ok1 ? 16u : 0u);
+            if (!both && rh) return;
+            const int sl = (v + rh) & (kRingSlots - 1);
+#pragma unroll
+            for (int i = 0; i < NCP; ++i) {
+                const int o = (q >> 1) + i * (Q / 2);
+                const int pr = v + rh + ((X - o) >> 1);
+                const bool ok = (unsigned)pr < (unsigned)npairs;
+                // branch-free: a pair outside the row becomes a zero-filled copy of nothing (never read)
+                cp_async16_zfill(ringb + o * kRingSlots + sl, tabb + rcopy[i] + (ok ? pr : 0) * 16, ok ? 16u : 0u);
+            }
         };
         // BULK: the pairs of ring iterations v and v + 1 (v even; v + 1 only while <= vlast) of outputs
         // q and q + 4, one bulk copy per output into the two adjacent slots.  Pairs outside the row
@@ -332,7 +367,7 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                 const bool ok1 = v + 1 <= vlast && (unsigned)(p0 + 1) < (unsigned)npairs;
                 const int first = ok0 ? 0 : 1;
                 nb[o] = (ok0 ? 16u : 0u) + (ok1 ? 16u : 0u);
-                src[o] = tabb + (o ? roff1 : roff0) + (long long)(p0 + first) * 16;
+                src[o] = tabb + roff[o < NO ? o : 0] + (long long)(p0 + first) * 16;
                 dst[o] = ringb + (q + o * Q) * kRingSlots + (v & (kRingSlots - 1)) + first;
             }
             mbar_arrive_expect_tx(bar, nb[0] + nb[1]);
@@ -360,7 +395,9 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                 ring_chunk(-4, -1);
                 ring_chunk(-2, -1);
             } else {
-                for (int u = -(X / 2); u < 0; ++u) ring_copy(u);
+                spread_rows();
+                ring_pair(-4, true);
+                ring_pair(-2, true);
             }
             if (STAGE) {
                 if (a.nextrap > 1) stage_idx(1);
@@ -381,26 +418,26 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
             }
             __syncwarp();  // control flow is warp-uniform here
             const long long pe = prow0 + (long long)l * a.nx;
-            float cur_s0 = 0.f, cur_c0 = 0.f, cur_s1 = 0.f, cur_c1 = 0.f;
+            float cur_s[NO] = {}, cur_c[NO] = {};
             if (!STAGE) {
                 // this step's Kahan values and the next step's operator indices: the loads are
                 // issued here and complete during the tap loop
-                if (img0) {
-                    cur_s0 = a.partial[pe];
-                    cur_c0 = a.comp[pe];
-                }
-                if (img1) {
-                    cur_s1 = a.partial[pe + Q];
-                    cur_c1 = a.comp[pe + Q];
-                }
+#pragma unroll
+                for (int o = 0; o < NO; ++o)
+                    if (imgo[o]) {
+                        cur_s[o] = a.partial[pe + o * Q];
+                        cur_c[o] = a.comp[pe + o * Q];
+                    }
                 if (l + 1 < a.nextrap) {
                     const uint16_t *inext = idx_j + (long long)(l + 1) * a.idx_lstride;
-                    nidx01 = (unsigned)inext[xq0] | ((unsigned)inext[xq1] << 16);
+                    nidx = 0;
+#pragma unroll
+                    for (int o = 0; o < NO; ++o) nidx |= (unsigned)inext[xq[o]] << (16 * o);
                 }
             }
             // the partial-image rows of the next step into L2 (read at the end of this step by the
             // stage, or at the start of the next one)
-            if (q == 0 && img0 && l + 1 < a.nextrap) {
+            if (q == 0 && imgo[0] && l + 1 < a.nextrap) {
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(a.partial + pe + a.nx));
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(a.comp + pe + a.nx));
             }
@@ -411,12 +448,18 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                 for (int e = 0; e < 8; ++e) acc[jj][e] = 0.f;
             if (warp_active) {  // warps past the CTA's share of the window skip the step's work
             float4 tp[X];
-            // input t: row srow0 + t, columns wide_col(row, q, 0/1)
+            // input t: row srow0 + t, columns wide_col<Q>(row, q, 0/1)
             auto load_in = [&](int row, float4 &va, float4 &vb) {
-                const float4 *r = ext + (size_t)row * G + 2 * q;
-                const int sw = (row >> 3) & 1;
-                va = r[sw];
-                vb = r[sw ^ 1];
+                if (Q == 8) {
+                    const float4 *r = ext + (size_t)row * G + q;
+                    va = r[0];
+                    vb = r[8];
+                } else {
+                    const float4 *r = ext + (size_t)row * G + 2 * q;
+                    const int sw = (row >> 3) & 1;
+                    va = r[sw];
+                    vb = r[sw ^ 1];
+                }
             };
 
             // prologue: t = 0 .. X-2, outputs jj <= t are active
@@ -435,12 +478,12 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                         wide_mac<ARITH>(acc[jj], fr, fi, va, vb);
                     }
                 }
-                // after t = 2u the slot of iteration u - 4 has been read; copy iteration u
-                if ((t & 1) == 0 && (t >> 1) < 3) {
+                // the slots of iterations -4 and -3 have been read: copy iterations 0 and 1
+                if (t == 2) {
                     if (BULK) {
-                        if (t == 2) ring_chunk(0, nmid + 3);
+                        ring_chunk(0, nmid + 3);
                     } else {
-                        ring_copy(t >> 1);
+                        ring_pair(0, true);
                         cp_async_commit();
                     }
                 }
@@ -449,18 +492,18 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
             int row = srow0 + X - 1;
             for (int u = 0; u < nmid; ++u, row += 2) {
                 const float4 *rs = ringb + (u & (kRingSlots - 1));
-                // iteration u - 1 has read the slot of iteration u + 3; wait for iteration u
-                if (BULK) {
-                    if (!(u & 1)) {
+                // iterations u - 2 and u - 1 have read the slots of u + 2 and u + 3; wait for u and u + 1
+                if (!(u & 1)) {
+                    if (BULK) {
                         ring_chunk(u + 2, nmid + 3);
                         chunk_wait();
+                    } else {
+                        ring_pair(u + 2, true);
+                        cp_async_commit();
+                        cp_async_wait<1>();
                     }
-                } else {
-                    ring_copy(u + 3);
-                    cp_async_commit();
-                    cp_async_wait<3>();
+                    __syncwarp();  // control flow is warp-uniform here
                 }
-                __syncwarp();  // control flow is warp-uniform here
                 {
                     float4 va, vb;
                     load_in(row, va, vb);
@@ -488,25 +531,19 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
             if (BULK) {
                 ring_chunk((nmid + 3) & ~1, nmid + 3);
             } else {
-                ring_copy(nmid + 3);
+                // for odd nmid iteration nmid + 4, whose slot iteration nmid has yet to read, does not exist
+                ring_pair((nmid + 3) & ~1, !(nmid & 1));
                 cp_async_commit();
             }
 #pragma unroll
             for (int e = 0; e < X - 1; ++e) {
                 float4 va, vb;
                 load_in(srow0 + L + e, va, vb);
-                if ((e & 1) == 0) {
-                    // steps e and e + 1 read iteration nmid + e / 2; later iterations may be in flight
-                    if (BULK) {
-                        if (!((nmid + (e >> 1)) & 1)) chunk_wait();
-                    } else {
-                        switch (e >> 1) {
-                            case 0: cp_async_wait<3>(); break;
-                            case 1: cp_async_wait<2>(); break;
-                            case 2: cp_async_wait<1>(); break;
-                            default: cp_async_wait<0>(); break;
-                        }
-                    }
+                // steps e and e + 1 read iteration nmid + e / 2; the last two chunks may be in flight
+                if ((e & 1) == 0 && !((nmid + (e >> 1)) & 1)) {
+                    if (BULK) chunk_wait();
+                    else if (e < 4) cp_async_wait<1>();
+                    else cp_async_wait<0>();
                     __syncwarp();  // control flow is warp-uniform here
                 }
 #pragma unroll
@@ -539,8 +576,8 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                     if (x < MP) {
                         const int prow = NC + MP + x;
                         const unsigned ra = map_rank(dst + (size_t)x * G, crank - 1);
-                        st_cluster(ra + wide_col(prow, q, 0) * 16, make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]));
-                        st_cluster(ra + wide_col(prow, q, 1) * 16, make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]));
+                        st_cluster(ra + wide_col<Q>(prow, q, 0) * 16, make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]));
+                        st_cluster(ra + wide_col<Q>(prow, q, 1) * 16, make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]));
                     }
                 }
             }
@@ -551,8 +588,8 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                     const int x = b * X + jj - (NC - MP);
                     if (x >= 0) {
                         const unsigned ra = map_rank(dst + (size_t)x * G, crank + 1);
-                        st_cluster(ra + wide_col(x, q, 0) * 16, make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]));
-                        st_cluster(ra + wide_col(x, q, 1) * 16, make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]));
+                        st_cluster(ra + wide_col<Q>(x, q, 0) * 16, make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]));
+                        st_cluster(ra + wide_col<Q>(x, q, 1) * 16, make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]));
                     }
                 }
             }
@@ -565,19 +602,17 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
             // every ring slot has been read: copy the next step's prologue pairs (u < 0) now, so
             // that they arrive during the halo exchange and the imaging
             if (warp_active && l + 1 < a.nextrap) {
-                if (STAGE) {
-                    const unsigned w0 = sst[0], w1 = sst[1];
-                    roff0 = ((w0 >> (16 * (xq0 & 1))) & 0xffffu) * (unsigned)row_bytes;
-                    roff1 = ((w1 >> (16 * (xq1 & 1))) & 0xffffu) * (unsigned)row_bytes;
-                } else {
-                    roff0 = (nidx01 & 0xffffu) * (unsigned)row_bytes;
-                    roff1 = (nidx01 >> 16) * (unsigned)row_bytes;
-                }
+#pragma unroll
+                for (int o = 0; o < NO; ++o)
+                    roff[o] = (STAGE ? (sst[o] >> (16 * (xq[o] & 1))) & 0xffffu : (nidx >> (16 * o)) & 0xffffu) *
+                              (unsigned)row_bytes;
                 if (BULK) {
                     ring_chunk(-4, -1);
                     ring_chunk(-2, -1);
                 } else {
-                    for (int u = -(X / 2); u < 0; ++u) ring_copy(u);
+                    spread_rows();
+                    ring_pair(-4, true);
+                    ring_pair(-2, true);
                 }
                 // the words just read are refilled for step l + 2 (their reads are complete: the
                 // copies above used them)
@@ -590,8 +625,8 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
             for (int jj = 0; jj < X; ++jj) {
                 const int prow = b * X + MP + jj;
                 float4 *dst = ext + (size_t)prow * G;
-                dst[wide_col(prow, q, 0)] = make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]);
-                dst[wide_col(prow, q, 1)] = make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]);
+                dst[wide_col<Q>(prow, q, 0)] = make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]);
+                dst[wide_col<Q>(prow, q, 1)] = make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]);
             }
             // Re(S conj R) of both slots per output, summed over the group's 4 lanes by a reduce-scatter:
             // exchange across lanes q ^ 2 keeps the 4 outputs with (jj & 2) == (q & 2), exchange
@@ -614,41 +649,53 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                 }
                 img[jj] = ia + ib;
             }
-            const bool hi2 = (q & 2) != 0, hi1 = (q & 1) != 0;
-            float r4[4];  // outputs {0, 1, 4, 5} ^ (q & 2)
+            // a reduce-scatter: each exchange halves the outputs a lane keeps, until q + o Q are left
+            float img_q[NO];
+            if constexpr (Q == 8) {
+                const bool hi4 = (q & 4) != 0, hi2 = (q & 2) != 0, hi1 = (q & 1) != 0;
+                float r4[4], r2[2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int base = (i & 1) | ((i & 2) << 1);
-                const float keep = hi2 ? img[base ^ 2] : img[base];
-                const float send = hi2 ? img[base] : img[base ^ 2];
-                r4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-            }
-            float img_q[2];  // outputs q and q + 4
+                for (int i = 0; i < 4; ++i) {
+                    const float keep = hi4 ? img[i + 4] : img[i], send = hi4 ? img[i] : img[i + 4];
+                    r4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+                }
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const float keep = hi1 ? r4[2 * k + 1] : r4[2 * k];
-                const float send = hi1 ? r4[2 * k] : r4[2 * k + 1];
-                img_q[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+                for (int i = 0; i < 2; ++i) {
+                    const float keep = hi2 ? r4[i + 2] : r4[i], send = hi2 ? r4[i] : r4[i + 2];
+                    r2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+                }
+                const float keep = hi1 ? r2[1] : r2[0], send = hi1 ? r2[0] : r2[1];
+                img_q[0] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+            } else {
+                const bool hi2 = (q & 2) != 0, hi1 = (q & 1) != 0;
+                float r4[4];  // outputs {0, 1, 4, 5} ^ (q & 2)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int base = (i & 1) | ((i & 2) << 1);
+                    const float keep = hi2 ? img[base ^ 2] : img[base];
+                    const float send = hi2 ? img[base] : img[base ^ 2];
+                    r4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+                }
+#pragma unroll
+                for (int k = 0; k < NO; ++k) {
+                    const float keep = hi1 ? r4[2 * k + 1] : r4[2 * k];
+                    const float send = hi1 ? r4[2 * k] : r4[2 * k + 1];
+                    img_q[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+                }
             }
-            const float img_q0 = img_q[0], img_q1 = img_q[1];
             // Kahan update (the operations of kahan_add) on the values loaded at the step's start
-            if (STAGE) {
-                cur_s0 = __uint_as_float(sst[2]);
-                cur_c0 = __uint_as_float(sst[3]);
-                cur_s1 = __uint_as_float(sst[4]);
-                cur_c1 = __uint_as_float(sst[5]);
-            }
-            if (img0) {
-                const float y = img_q0 - cur_c0;
-                const float t = cur_s0 + y;
-                a.partial[pe] = t;
-                a.comp[pe] = (t - cur_s0) - y;
-            }
-            if (img1) {
-                const float y = img_q1 - cur_c1;
-                const float t = cur_s1 + y;
-                a.partial[pe + Q] = t;
-                a.comp[pe + Q] = (t - cur_s1) - y;
+#pragma unroll
+            for (int o = 0; o < NO; ++o) {
+                if (STAGE) {
+                    cur_s[o] = __uint_as_float(sst[NO + 2 * o]);
+                    cur_c[o] = __uint_as_float(sst[NO + 2 * o + 1]);
+                }
+                if (imgo[o]) {
+                    const float y = img_q[o] - cur_c[o];
+                    const float t = cur_s[o] + y;
+                    a.partial[pe + o * Q] = t;
+                    a.comp[pe + o * Q] = (t - cur_s[o]) - y;
+                }
             }
             if (STAGE && l + 1 < a.nextrap) stage_kahan(l + 1);  // refilled for the next step
             }  // warp_active
@@ -671,8 +718,8 @@ __global__ void __launch_bounds__(WideShape::NW * 32, 1) migrate_wide_kernel(Mig
                 const int sq = sg.y & (Q - 1), sh = sg.y / Q;
                 for (int x = lo + (int)threadIdx.x; x < hi; x += blockDim.x) {
                     const int pos = x - c0 + MP;
-                    const float *fa = extf + ((size_t)pos * G + wide_col(pos, sq, 0)) * 4;
-                    const float *fb = extf + ((size_t)pos * G + wide_col(pos, sq, 1)) * 4;
+                    const float *fa = extf + ((size_t)pos * G + wide_col<Q>(pos, sq, 0)) * 4;
+                    const float *fb = extf + ((size_t)pos * G + wide_col<Q>(pos, sq, 1)) * 4;
                     ws[x - r0] = cpx{fa[sh], fa[2 + sh]};
                     rs[x - r0] = cpx{fb[sh], -fb[2 + sh]};
                 }
