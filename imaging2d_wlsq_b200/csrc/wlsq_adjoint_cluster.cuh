@@ -239,7 +239,10 @@ __global__ void __launch_bounds__(kDcNW * 32, 1) demigrate_cluster_kernel(Demigr
         const int2 item = a.items[it];
         const GroupDesc grp = a.groups[item.x];
         const int j = item.y, u0 = grp.u0, W = grp.W;
-        const int base = u0 + c0;  // model position of local position 0
+        // model position of local position 0.  A CTA past the end of a narrow group's window (c0 >= W) has
+        // no outputs, but its operator rows are still looked up: its base stays inside the model, or the
+        // staged index row would be empty and the rows read at whatever shared memory holds before it.
+        const int base = min(u0 + c0, a.nx - 1);
         const uint16_t *idx_j = a.idx + (long long)j * a.idx_jstride;
         float4 *ckpt = a.ckpt_mode != 0
                            ? reinterpret_cast<float4 *>(a.ckpt_items) + ((long long)it * csize + crank) * a.nslab * pe
