@@ -956,8 +956,10 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             wf = stage ? migrate_wide_kernel<1, true, true> : migrate_wide_kernel<1, false, true>;
         else if (flags & IMG2D_FLAG_WIDE_SCALAR)
             wf = stage ? migrate_wide_kernel<0, true> : migrate_wide_kernel<0, false>;
+        else if (cluster2_mp(M) > 64)
+            return false;  // a warp's 64 positions cover the operator's reach at every length that fits
         else
-            wf = stage ? migrate_wide_kernel<1, true> : migrate_wide_kernel<1, false>;
+            wf = stage ? migrate_wide_kernel<1, true, false, 4, true> : migrate_wide_kernel<1, false, false, 4, true>;
         const size_t smemw = (stage ? wide_stage_smem_bytes(M) : wide_smem_bytes(M)) + bars;
         if (smemw + static_reserve > (size_t)smem_optin) return false;
         int widest = make_groups(WideShape::G);
@@ -1066,7 +1068,9 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         const bool stage = wide_stage_smem_bytes<Wide16Shape>(M) + static_reserve <= (size_t)smem_optin;
         const size_t smemw = stage ? wide_stage_smem_bytes<Wide16Shape>(M) : wide_smem_bytes<Wide16Shape>(M);
         if (smemw + static_reserve > (size_t)smem_optin) return false;
-        KernelFn wf = stage ? migrate_wide_kernel<1, true, false, 8> : migrate_wide_kernel<1, false, false, 8>;
+        // up to 65 taps a warp's 32 positions cover the operator's reach: waits for neighbours only
+        if (cluster2_mp(M) > 32) return false;
+        KernelFn wf = stage ? migrate_wide_kernel<1, true, false, 8, true> : migrate_wide_kernel<1, false, false, 8, true>;
         const int widest = make_groups(Wide16Shape::G);
         const int K = (widest + Wide16Shape::PC - 1) / Wide16Shape::PC;
         if (!(K <= 8 || (K <= kMaxCluster && clusters_that_fit((const void *)wf, K, Wide16Shape::NW * 32, smemw) > 0)))

@@ -25,18 +25,25 @@
 // it as packed f32x2 FMAs (FFMA2: two lanes of work per instruction), ARITH = 0 as scalar FMAs.
 //
 // Operator taps reach the tap loop through the per-lane-group shared-memory ring of the cluster2
-// ring variant: lane q owns outputs q and q+4 of its group's block and copies their tap pairs with
-// 16-byte cp.async three tap-loop iterations before they are read.  The next depth step's operator
+// ring variant, copied with 16-byte cp.async two to three tap-loop iterations before they are read.  The next depth step's operator
 // indices and this step's Kahan partial-image values of those two positions reach the thread
 // through a per-thread shared-memory stage filled by cp.async a step ahead (STAGE, where the
 // shared memory allows), or are loaded into registers at the start of the step.  The BULK variant
 // fills the same ring with 1-D bulk copies completing on per-warp transaction-count barriers.
 //
 // Per depth step: tap loop into registers; aperture mask; edge outputs pushed into the neighbour's
-// halo staging (distributed shared memory, double-buffered by step parity); cluster barrier arrive
-// (release of the pushes); the next step's first tap pairs copied; __syncthreads;
-// in-place write; imaging (Re(S conj R), shuffle over the group's 4 lanes, Kahan update of the
-// CTA's private partial row); cluster barrier wait; halo copy; __syncthreads.
+// halo staging (distributed shared memory, double-buffered by step parity); the next step's first tap
+// pairs copied; in-place write; imaging (Re(S conj R), shuffle over the group's 4 lanes, Kahan update
+// of the CTA's private partial row); halo copy.  Warps wait for their two neighbours only (DF, below).
+//
+// Measured on a B200 against barriers of the CTA and the cluster in every step (FMA pipe 53% busy, 64%
+// now): 256 uneven shots of 2048 x 80, 128 frequencies, 35 taps 47.1 -> 43.1 ms; 64 shots of 4096 x 30,
+// 64 frequencies, 55 taps 13.2 -> 12.1 ms.
+//
+// Eight lanes per group (LANES = 8) give the 16-slot shape, 16 slots x 512 positions per CTA: each
+// operator row feeds twice the multiply-adds.  It is the default where its clusters fill the GPU: 32
+// shots of 1024 x 60, 256 frequencies, 31 taps 6.65 ms with migrate_cluster2_kernel's scalar FMAs,
+// 6.39 ms with packed ones, 5.78 ms without the barriers.
 #pragma once
 #include "wlsq_cluster2.cuh"
 
@@ -123,6 +130,30 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned 
     return done != 0;
 }
 
+// plain arrival (release) on a barrier of this CTA
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
+{
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// arrival on a barrier of another CTA of the cluster (address from map_rank), releasing at cluster
+// scope what this thread (and, after a __syncwarp, its warp) wrote there
+__device__ __forceinline__ void mbar_arrive_cluster(unsigned addr)
+{
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try_wait_cluster(unsigned long long *bar, unsigned parity)
+{
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // 1-D bulk copy global -> this CTA's shared memory, completing bytes on the barrier (no multicast)
 __device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
 {
@@ -175,14 +206,27 @@ __device__ __forceinline__ void wide_mac(float (&c)[8], float fr, float fi, cons
 // chunk completing on one of two transaction-count barriers of the warp (alternating), where the
 // cp.async ring would wait for a commit group.  A chunk is issued where the cp.async ring copies
 // its later iteration and waited for where the ring waits for its first one.
-template <int ARITH, bool STAGE, bool BULK = false, int LANES = 4>
+//
+// DF: no barrier of the CTA or the cluster inside the depth loop.  A warp's outputs need only its
+// neighbours' rows (M <= the 8 P positions of a warp), so it waits for those two warps alone: before
+// writing its rows in place, until they have read step l (barrier rd of the warp, two arrivals), and
+// before reading step l + 1, until they have written theirs (wr).  At the edges of the CTA the pushed
+// halo and an arrival from the neighbouring CTA's edge warp (hb) take the place of the neighbour; the
+// edge warp copies the halo from the staging itself.  The staging of a parity is pushed again only
+// after the pusher has received this CTA's push of the step between, which follows the copy; a pusher
+// may be one step ahead, so even and odd exchanges have a barrier each.  rd and wr need only one: a
+// neighbour's next arrival follows what this warp does after its wait.  With
+// barriers every warp does its step-boundary work (writes, imaging, copies: a quarter of the step) at
+// the same time and the FMA pipe idles; this way the warps of an SM sub-partition drift apart and one's
+// boundary work runs beside the others' tap loops.  Every wait has a limit, like BULK's.
+template <int ARITH, bool STAGE, bool BULK = false, int LANES = 4, bool DF = false>
 __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_kernel(MigrateArgs a)
 {
     using S = WideShapeQ<LANES>;
     constexpr int Q = S::Q, G = S::G, P = S::P, X = S::X, PC = S::PC;
     constexpr int NO = X / Q;  // outputs whose operator row, index and Kahan values a lane looks after
     constexpr int SW = wide_stage_words<S>();
-    static_assert(!BULK || Q == 4, "the bulk-copy ring is built on 4 lanes per group");
+    static_assert(!BULK || (Q == 4 && !DF), "the bulk-copy ring is built on 4 lanes per group and CTA barriers");
     const int M = a.M, L = 2 * a.M + 1;
     const int MP = cluster2_mp(M);
     const int NEXT = PC + 2 * MP;
@@ -217,6 +261,28 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
         }
         __syncwarp();
     }
+    // DF: barriers of each warp and of the two edges, the phases this warp has waited for
+    __shared__ unsigned long long s_rd[DF ? S::NW : 1], s_wr[DF ? S::NW : 1], s_hb[4];
+    unsigned n_rd = 0, n_wr = 0, hb_base = 0;
+    bool wait_failed = false;
+    if (DF && threadIdx.x < S::NW) {
+        mbar_init(s_rd + threadIdx.x, 2);
+        mbar_init(s_wr + threadIdx.x, 2);
+        if (threadIdx.x < 4) mbar_init(s_hb + threadIdx.x, 1);
+        mbar_init_fence();  // made visible to the cluster by the first item's barriers
+    }
+    auto df_wait = [&](unsigned long long *bar, unsigned phase, bool cluster) {
+        auto ready = [&]() { return cluster ? mbar_try_wait_cluster(bar, phase & 1) : mbar_try_wait(bar, phase & 1); };
+        if (wait_failed || ready()) return;
+        const long long t0 = clock64();
+        while (!ready()) {
+            if (clock64() - t0 > 2 * kBulkWaitCycles) {
+                wait_failed = true;
+                if (a.status) atomicOr(a.status, 2);
+                break;
+            }
+        }
+    };
     const unsigned rank0_item = map_rank(&s_item, 0);
     const int row_bytes = a.tab_stride * 8;
     // register budget (512 threads at <= 128 registers): the partial-image, table and owner
@@ -405,11 +471,39 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
             }
         }
         cp_async_commit();
+        // DF: the warps whose rows this one shares (itself where there is none: the barriers expect two)
+        const int last_warp = NC / (P * X) - 1;
+        const int wl = max(warp - 1, 0), wr = min(warp + 1, last_warp);
+        const bool hb_left = DF && warp == 0 && crank > 0, hb_right = DF && warp == last_warp && crank + 1 < csize;
+        auto df_signal = [&](unsigned long long *bars) {
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(bars + wl);
+                mbar_arrive(bars + wr);
+            }
+        };
         const int srow0 = b * X + MP - M;  // row of input t = 0
         const int nmid = (L - X + 1) / 2;  // middle tap-loop iterations (two inputs each)
 
-        for (int l = 0; l < a.nextrap; ++l) {
+        for (int l = 0; l < a.nextrap && (!DF || warp_active); ++l) {
             const int par = l & 1;
+            if (DF && l > 0) {
+                // the neighbours' rows of this step, or the halo pushed by the neighbouring CTA
+                df_wait(s_wr + warp, n_wr++, false);
+                if (hb_left || hb_right) {
+                    const unsigned ex = hb_base + l - 1;  // exchange number: its barriers, their phase
+                    const float4 *hs = stg + (size_t)(par * 2) * MP * G;
+                    if (hb_left) {
+                        df_wait(s_hb + (ex & 1), ex >> 1, true);
+                        for (int i = lane; i < MP * G; i += 32) ext[i] = hs[i];
+                    }
+                    if (hb_right) {
+                        df_wait(s_hb + 2 + (ex & 1), ex >> 1, true);
+                        for (int i = lane; i < MP * G; i += 32) ext[(NC + MP) * G + i] = hs[MP * G + i];
+                    }
+                    __syncwarp();
+                }
+            }
             // this step's prologue pairs (copied at the end of the previous step) for the group
             cp_async_wait_all();
             if (BULK && warp_active) {
@@ -558,6 +652,7 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
                     }
                 }
             }
+            if (DF) df_signal(s_rd);  // this warp has read its neighbours' rows of step l
             // outputs outside every shot aperture of their slot stay zero; most lanes have none
             if ((in_a & in_b) != (1u << X) - 1u) {
 #pragma unroll
@@ -593,12 +688,20 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
                     }
                 }
             }
+            if (DF && l + 1 < a.nextrap && (hb_left || hb_right)) {
+                __syncwarp();
+                // the right edge of the CTA to the left, the left edge of the CTA to the right
+                if (lane == 0) {
+                    if (hb_left) mbar_arrive_cluster(map_rank(s_hb + 2 + ((hb_base + l) & 1), crank - 1));
+                    if (hb_right) mbar_arrive_cluster(map_rank(s_hb + ((hb_base + l) & 1), crank + 1));
+                }
+            }
             }  // warp_active
             // The neighbours read only their halo staging (the pushes above), never this CTA's ext[]:
             // arrive now, so the barrier's release covers the pushes but not the in-place writes.
             // The staging of parity par^1 is rewritten (step l+2) only after this CTA's arrival of
             // step l+1, which follows its copy of that staging at the end of this step.
-            cluster_arrive();
+            if (!DF) cluster_arrive();
             // every ring slot has been read: copy the next step's prologue pairs (u < 0) now, so
             // that they arrive during the halo exchange and the imaging
             if (warp_active && l + 1 < a.nextrap) {
@@ -619,15 +722,25 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
                 if (STAGE && l + 2 < a.nextrap) stage_idx(l + 2);
             }
             cp_async_commit();
-            __syncthreads();  // every read of step l's values in ext[] is done
-            if (warp_active) {
+            // in place, once every read of step l's values in this warp's rows of ext[] is done
+            auto write_rows = [&]() {
 #pragma unroll
-            for (int jj = 0; jj < X; ++jj) {
-                const int prow = b * X + MP + jj;
-                float4 *dst = ext + (size_t)prow * G;
-                dst[wide_col<Q>(prow, q, 0)] = make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]);
-                dst[wide_col<Q>(prow, q, 1)] = make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]);
+                for (int jj = 0; jj < X; ++jj) {
+                    const int prow = b * X + MP + jj;
+                    float4 *dst = ext + (size_t)prow * G;
+                    dst[wide_col<Q>(prow, q, 0)] = make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]);
+                    dst[wide_col<Q>(prow, q, 1)] = make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]);
+                }
+            };
+            if (DF) {
+                df_wait(s_rd + warp, n_rd++, false);
+                write_rows();
+                if (l + 1 < a.nextrap) df_signal(s_wr);
+            } else {
+                __syncthreads();
             }
+            if (warp_active) {
+            if (!DF) write_rows();
             // Re(S conj R) of both slots per output, summed over the group's 4 lanes by a reduce-scatter:
             // exchange across lanes q ^ 2 keeps the 4 outputs with (jj & 2) == (q & 2), exchange
             // across q ^ 1 keeps jj = q and q + 4 (6 shuffles instead of 8 x 2)
@@ -700,6 +813,7 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
             if (STAGE && l + 1 < a.nextrap) stage_kahan(l + 1);  // refilled for the next step
             }  // warp_active
             if (STAGE) cp_async_commit();  // the Kahan words, waited for at the next step's start
+            if (DF) continue;
             cluster_wait();
             const float4 *hs = stg + (size_t)((par ^ 1) * 2) * MP * G;
             for (int i = threadIdx.x; i < 2 * MP * G; i += blockDim.x) {
@@ -707,6 +821,10 @@ __global__ void __launch_bounds__(WideShapeQ<LANES>::NW * 32, 1) migrate_wide_ke
                 ext[(side ? (NC + MP) * G : 0) + r] = hs[i];
             }
             __syncthreads();
+        }
+        if (DF) {
+            hb_base += a.nextrap - 1;
+            __syncthreads();  // every warp's rows of the last step are written
         }
         if (a.write_back) {
             for (int k = grp.seg_begin; k < grp.seg_begin + grp.nseg; ++k) {
