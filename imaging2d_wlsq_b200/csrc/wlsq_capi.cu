@@ -10,6 +10,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/imaging2d_wlsq_b200.h"
@@ -409,19 +410,159 @@ static size_t alloc_limit()
     return g_alloc_limit;
 }
 
-static int device_alloc(void **p, size_t n)
+// Device blocks given back by plans and host calls, kept for the next allocation of about their size (up
+// to 2 GB a device; img2d_release_host_cache frees them, and so does an allocation that finds no
+// memory).  cudaMalloc and cudaFree of the large buffers cost milliseconds: the planes of a
+// demigration of 5 shots (0.6 GB) 13 ms, the tables of a dense call (0.25 GB) 3 ms.  A block enters
+// only after the device has finished its work (cudaFree waits for the same), so whoever takes it, on
+// any stream or thread, finds nobody using it.
+constexpr size_t kPoolMaxBytes = 2ull << 30, kPoolMinBlock = 256 << 10;
+struct DevicePool {
+    std::mutex mu;
+    std::map<int, std::multimap<size_t, void *>> blocks;  // per device, by size
+    std::map<int, size_t> bytes;
+};
+static DevicePool &device_pool()
+{
+    static DevicePool *pool = new DevicePool;  // never destroyed: static objects give buffers back at exit
+    return *pool;
+}
+
+static void pool_flush(int dev)
+{
+    DevicePool &pool = device_pool();
+    std::lock_guard<std::mutex> lock(pool.mu);
+    for (auto &b : pool.blocks[dev]) cudaFree(b.second);
+    pool.blocks[dev].clear();
+    pool.bytes[dev] = 0;
+}
+
+// n bytes on the current device; *got: the size of the block, for device_free.
+static int device_alloc(void **p, size_t n, size_t *got, int *dev)
 {
     *p = nullptr;
+    *got = n;
+    *dev = 0;
     const size_t lim = alloc_limit();
     if (lim && n > lim)
         return fail(IMG2D_ENOMEM, "device allocation of " + std::to_string(n) + " bytes refused: above the " +
                                       std::to_string(lim) + "-byte allocation limit (IMG2D_ALLOC_LIMIT_BYTES)");
+    if (cudaGetDevice(dev) != cudaSuccess) cudaGetLastError();
+    if (n >= kPoolMinBlock) {
+        DevicePool &pool = device_pool();
+        std::lock_guard<std::mutex> lock(pool.mu);
+        auto &blocks = pool.blocks[*dev];
+        auto it = blocks.lower_bound(n);
+        if (it != blocks.end() && it->first <= n + n / 4) {
+            *p = it->second;
+            *got = it->first;
+            pool.bytes[*dev] -= it->first;
+            blocks.erase(it);
+            return IMG2D_OK;
+        }
+    }
     cudaError_t e = cudaMalloc(p, n);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        pool_flush(*dev);
+        e = cudaMalloc(p, n);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
         return fail(IMG2D_ENOMEM, "cudaMalloc(" + std::to_string(n) + " bytes): " + cudaGetErrorString(e));
     }
+    return IMG2D_OK;
+}
+
+static void device_free(void *p, size_t n, int dev)
+{
+    int cur = -1;
+    if (n >= kPoolMinBlock && n <= kPoolMaxBytes && cudaGetDevice(&cur) == cudaSuccess && cur == dev &&
+        cudaDeviceSynchronize() == cudaSuccess) {
+        DevicePool &pool = device_pool();
+        std::lock_guard<std::mutex> lock(pool.mu);
+        if (pool.bytes[dev] + n <= kPoolMaxBytes) {
+            pool.blocks[dev].emplace(n, p);
+            pool.bytes[dev] += n;
+            return;
+        }
+    }
+    cudaGetLastError();
+    cudaFree(p);
+}
+
+// Pinned staging for uploads from pageable memory.  A plain cudaMemcpy of pageable memory runs at the
+// speed of one host thread (about 10 GB/s here); eight workers copying 4 MB pieces into a pinned ring,
+// each sending its own, keep the link busy.  One upload uses the ring at a time, others take the plain
+// copy.  The ring (64 MB) is kept until img2d_release_host_cache.
+constexpr size_t kStagePiece = 4 << 20;
+constexpr int kStageWorkers = 8;
+struct StageRing {
+    std::mutex mu;
+    unsigned char *host = nullptr;
+};
+static StageRing &stage_ring()
+{
+    static StageRing *r = new StageRing;
+    return *r;
+}
+
+// Host to device on stream st; returns when the copy has completed.
+static int upload(void *dst, const void *src, size_t n, cudaStream_t st)
+{
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    StageRing &ring = stage_ring();
+    std::unique_lock<std::mutex> lock(ring.mu, std::defer_lock);
+    if (n < 4 * kStagePiece || !pageable || !lock.try_lock()) {
+        IMG2D_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
+        IMG2D_CUDA(cudaStreamSynchronize(st));
+        return IMG2D_OK;
+    }
+    if (!ring.host && cudaHostAlloc((void **)&ring.host, 2 * kStageWorkers * kStagePiece, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        ring.host = nullptr;
+        IMG2D_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
+        IMG2D_CUDA(cudaStreamSynchronize(st));
+        return IMG2D_OK;
+    }
+    int dev = 0;
+    IMG2D_CUDA(cudaGetDevice(&dev));
+    std::atomic<size_t> next{0};
+    std::atomic<int> err{(int)cudaSuccess};
+    auto work = [&](int w) {
+        cudaError_t e = cudaSetDevice(dev);
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+        for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+        for (int k = 0; e == cudaSuccess && err.load() == (int)cudaSuccess; ++k) {
+            const size_t at = next.fetch_add(kStagePiece);
+            if (at >= n) break;
+            const size_t m = std::min(kStagePiece, n - at);
+            unsigned char *slot = ring.host + (size_t)(2 * w + (k & 1)) * kStagePiece;
+            if (k >= 2) e = cudaEventSynchronize(ev[k & 1]);  // the slot's previous piece has left
+            if (e != cudaSuccess) break;
+            std::memcpy(slot, (const unsigned char *)src + at, m);
+            e = cudaMemcpyAsync((unsigned char *)dst + at, slot, m, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = cudaEventRecord(ev[k & 1], st);
+        }
+        if (e != cudaSuccess) err.store((int)e);
+        for (cudaEvent_t x : ev)
+            if (x) cudaEventDestroy(x);
+    };
+    std::vector<std::thread> threads;
+    try {
+        const int workers = std::max(1, std::min<int>(kStageWorkers, (int)std::thread::hardware_concurrency() / 2));
+        threads.reserve(workers);
+        for (int w = 1; w < workers; ++w) threads.emplace_back(work, w);
+    } catch (...) {
+        // fewer workers (the caller alone does too)
+    }
+    work(0);
+    for (std::thread &t : threads) t.join();
+    IMG2D_CUDA(cudaStreamSynchronize(st));  // also before the ring has its next user
+    IMG2D_CUDA((cudaError_t)err.load());
     return IMG2D_OK;
 }
 
@@ -438,11 +579,12 @@ struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
     bool owned = false;
+    int dev = 0;               // device of an owned block
     Carver *carver = nullptr;  // when set, storage is carved from it and never freed
     ~DevBuf() { release(); }
     void release()
     {
-        if (p && owned) cudaFree(p);
+        if (p && owned) device_free(p, bytes, dev);
         p = nullptr;
         bytes = 0;
         owned = false;
@@ -462,10 +604,11 @@ struct DevBuf {
             return IMG2D_OK;
         }
         if (n == 0) n = 16;
-        const int rc = device_alloc(&p, n);
+        size_t got = 0;
+        const int rc = device_alloc(&p, n, &got, &dev);
         if (rc) return rc;
         owned = true;
-        bytes = n;
+        bytes = got;
         return IMG2D_OK;
     }
     template <class T> T *as() const { return static_cast<T *>(p); }
@@ -1241,7 +1384,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                                           " MiB of fixed scratch of the no-allocation entry point");
         p->grid = (int)std::min<size_t>((size_t)p->grid, fit);
     }
-    for (;;) {
+    while (mode != OP_DENSE) {  // dense calls take the images of the single shots only
         rc = p->partial.ensure((size_t)p->grid * plane * sizeof(float));
         if (!rc && (!p->rows || p->n_items > p->grid))  // one item per CTA needs no compensation
             rc = p->comp.ensure((size_t)p->grid * plane * sizeof(float));
@@ -1594,18 +1737,23 @@ static int demig_prepare(img2d_plan *p, int slab)
 
 // Scoped device allocation for the host entry points.
 struct Scratch {
-    std::vector<void *> ptrs;
+    struct Block {
+        void *p;
+        size_t bytes;
+        int dev;
+    };
+    std::vector<Block> blocks;
     ~Scratch()
     {
-        for (void *q : ptrs) cudaFree(q);
+        for (const Block &b : blocks) device_free(b.p, b.bytes, b.dev);
     }
     template <class T> int alloc(T **out, size_t n)
     {
-        void *q = nullptr;
-        const int rc = device_alloc(&q, n ? n : 16);
+        Block b{};
+        const int rc = device_alloc(&b.p, n ? n : 16, &b.bytes, &b.dev);
         if (rc) return rc;
-        ptrs.push_back(q);
-        *out = static_cast<T *>(q);
+        blocks.push_back(b);
+        *out = static_cast<T *>(b.p);
         return IMG2D_OK;
     }
 };
@@ -1658,10 +1806,10 @@ static int run_dense(int ns, int nextrap, int nz, int nx, int nf, int nt, int M,
     if ((rc = sc.alloc(&dW, wel * sizeof(cpx)))) return rc;
     if ((rc = sc.alloc(&dS, wel * sizeof(cpx)))) return rc;
     if ((rc = sc.alloc(&dI, (size_t)ns * plane * sizeof(float)))) return rc;
-    IMG2D_CUDA(cudaMemcpy(dF, opF, tab * sizeof(cpx), cudaMemcpyHostToDevice));
-    IMG2D_CUDA(cudaMemcpy(dB, opB, tab * sizeof(cpx), cudaMemcpyHostToDevice));
-    IMG2D_CUDA(cudaMemcpy(dW, wave, wel * sizeof(cpx), cudaMemcpyHostToDevice));
-    IMG2D_CUDA(cudaMemcpy(dS, shot, wel * sizeof(cpx), cudaMemcpyHostToDevice));
+    if ((rc = upload(dF, opF, tab * sizeof(cpx), 0))) return rc;
+    if ((rc = upload(dB, opB, tab * sizeof(cpx), 0))) return rc;
+    if ((rc = upload(dW, wave, wel * sizeof(cpx), 0))) return rc;
+    if ((rc = upload(dS, shot, wel * sizeof(cpx), 0))) return rc;
     MigrateArgs a = base_args(&plan, dW, dS);
     a.denseF = dF;
     a.denseB = dB;
@@ -2559,6 +2707,19 @@ void img2d_release_host_cache(void)
         delete kv.second.bufs;
     }
     g_host_cache.clear();
+    std::vector<int> devs;
+    {
+        DevicePool &pool = device_pool();
+        std::lock_guard<std::mutex> plock(pool.mu);
+        for (const auto &kv : pool.blocks) devs.push_back(kv.first);
+    }
+    for (int d : devs) pool_flush(d);
+    {
+        StageRing &ring = stage_ring();
+        std::lock_guard<std::mutex> rlock(ring.mu);
+        if (ring.host) cudaFreeHost(ring.host);
+        ring.host = nullptr;
+    }
     if (cur >= 0 && cudaSetDevice(cur) != cudaSuccess) cudaGetLastError();
 }
 
