@@ -3,10 +3,12 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <map>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -493,11 +495,11 @@ static void device_free(void *p, size_t n, int dev)
 }
 
 // Pinned staging for uploads from pageable memory.  A plain cudaMemcpy of pageable memory runs at the
-// speed of one host thread (about 10 GB/s here); eight workers copying 4 MB pieces into a pinned ring,
-// each sending its own, keep the link busy.  One upload uses the ring at a time, others take the plain
-// copy.  The ring (64 MB) is kept until img2d_release_host_cache.
-constexpr size_t kStagePiece = 4 << 20;
-constexpr int kStageWorkers = 8;
+// speed of one host thread (about 10 GB/s here); four workers copying 2 MB pieces into a pinned ring,
+// each sending its own, reach 34 GB/s (eight 31, sixteen 22).  One upload uses the ring at a time, others take the plain
+// copy.  The ring (16 MB) is kept until img2d_release_host_cache.
+constexpr size_t kStagePiece = 2 << 20;
+constexpr int kStageWorkers = 4;
 struct StageRing {
     std::mutex mu;
     unsigned char *host = nullptr;
@@ -508,61 +510,103 @@ static StageRing &stage_ring()
     return *r;
 }
 
-// Host to device on stream st; returns when the copy has completed.
-static int upload(void *dst, const void *src, size_t n, cudaStream_t st)
+// One piece of an upload; the pieces of group g are issued before those of group g + 1.
+struct UploadPiece {
+    void *dst;
+    const void *src;
+    size_t n;
+    int group;
+};
+
+static void add_pieces(std::vector<UploadPiece> &v, void *dst, const void *src, size_t n, int group)
 {
+    for (size_t at = 0; at < n; at += kStagePiece)
+        v.push_back({(unsigned char *)dst + at, (const unsigned char *)src + at, std::min(kStagePiece, n - at), group});
+}
+
+// Host to device on stream st.  ready(g) runs on the calling thread once every piece of group g is queued
+// on st; returns when all copies have completed.  The workers live for the whole call: a new thread's
+// first CUDA call costs a tenth of a millisecond, as much as two pieces.
+static int upload(const std::vector<UploadPiece> &pieces, int groups, cudaStream_t st, const std::function<int(int)> &ready)
+{
+    size_t total = 0;
+    for (const UploadPiece &u : pieces) total += u.n;
     cudaPointerAttributes at{};
-    const bool pageable = cudaPointerGetAttributes(&at, src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    bool staged = total >= 4 * kStagePiece &&
+                  (cudaPointerGetAttributes(&at, pieces[0].src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered);
     cudaGetLastError();
     StageRing &ring = stage_ring();
     std::unique_lock<std::mutex> lock(ring.mu, std::defer_lock);
-    if (n < 4 * kStagePiece || !pageable || !lock.try_lock()) {
-        IMG2D_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
-        IMG2D_CUDA(cudaStreamSynchronize(st));
-        return IMG2D_OK;
-    }
-    if (!ring.host && cudaHostAlloc((void **)&ring.host, 2 * kStageWorkers * kStagePiece, cudaHostAllocPortable) != cudaSuccess) {
+    staged = staged && lock.try_lock();
+    if (staged && !ring.host &&
+        cudaHostAlloc((void **)&ring.host, 2 * kStageWorkers * kStagePiece, cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
         ring.host = nullptr;
-        IMG2D_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
-        IMG2D_CUDA(cudaStreamSynchronize(st));
-        return IMG2D_OK;
+        staged = false;
     }
-    int dev = 0;
+    int dev = 0, rc = IMG2D_OK;
     IMG2D_CUDA(cudaGetDevice(&dev));
-    std::atomic<size_t> next{0};
-    std::atomic<int> err{(int)cudaSuccess};
+    std::mutex mu;
+    std::condition_variable cv;
+    std::vector<size_t> left(groups, 0);  // pieces of a group not yet queued
+    for (const UploadPiece &u : pieces) ++left[u.group];
+    size_t next = 0;
+    cudaError_t err = cudaSuccess;
     auto work = [&](int w) {
         cudaError_t e = cudaSetDevice(dev);
         cudaEvent_t ev[2] = {nullptr, nullptr};
         for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-        for (int k = 0; e == cudaSuccess && err.load() == (int)cudaSuccess; ++k) {
-            const size_t at = next.fetch_add(kStagePiece);
-            if (at >= n) break;
-            const size_t m = std::min(kStagePiece, n - at);
+        std::unique_lock<std::mutex> l(mu);
+        for (int k = 0; e == cudaSuccess && err == cudaSuccess && next < pieces.size(); ++k) {
+            const UploadPiece u = pieces[next++];
+            l.unlock();
             unsigned char *slot = ring.host + (size_t)(2 * w + (k & 1)) * kStagePiece;
             if (k >= 2) e = cudaEventSynchronize(ev[k & 1]);  // the slot's previous piece has left
-            if (e != cudaSuccess) break;
-            std::memcpy(slot, (const unsigned char *)src + at, m);
-            e = cudaMemcpyAsync((unsigned char *)dst + at, slot, m, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) {
+                std::memcpy(slot, u.src, u.n);
+                e = cudaMemcpyAsync(u.dst, slot, u.n, cudaMemcpyHostToDevice, st);
+            }
             if (e == cudaSuccess) e = cudaEventRecord(ev[k & 1], st);
+            l.lock();
+            if (e == cudaSuccess && --left[u.group] == 0) cv.notify_one();
         }
-        if (e != cudaSuccess) err.store((int)e);
+        if (e != cudaSuccess) err = e;
+        cv.notify_one();
+        l.unlock();
         for (cudaEvent_t x : ev)
             if (x) cudaEventDestroy(x);
     };
     std::vector<std::thread> threads;
-    try {
-        const int workers = std::max(1, std::min<int>(kStageWorkers, (int)std::thread::hardware_concurrency() / 2));
-        threads.reserve(workers);
-        for (int w = 1; w < workers; ++w) threads.emplace_back(work, w);
-    } catch (...) {
-        // fewer workers (the caller alone does too)
+    if (staged) {
+        try {
+            threads.reserve(kStageWorkers);
+            for (int w = 0; w < kStageWorkers; ++w) threads.emplace_back(work, w);
+        } catch (...) {
+            if (threads.empty()) staged = false;  // fewer workers do as well
+        }
     }
-    work(0);
+    size_t plain = 0;
+    for (int g = 0; g < groups && !rc; ++g) {
+        if (staged) {
+            std::unique_lock<std::mutex> l(mu);
+            cv.wait(l, [&]() { return left[g] == 0 || err != cudaSuccess; });
+            if (err != cudaSuccess) break;
+        } else {
+            for (; plain < pieces.size() && pieces[plain].group == g && err == cudaSuccess; ++plain)
+                err = cudaMemcpyAsync(pieces[plain].dst, pieces[plain].src, pieces[plain].n, cudaMemcpyHostToDevice, st);
+            if (err != cudaSuccess) break;
+        }
+        rc = ready(g);
+    }
+    if (rc) {
+        std::lock_guard<std::mutex> l(mu);
+        next = pieces.size();
+    }
     for (std::thread &t : threads) t.join();
-    IMG2D_CUDA(cudaStreamSynchronize(st));  // also before the ring has its next user
-    IMG2D_CUDA((cudaError_t)err.load());
+    const cudaError_t done = cudaStreamSynchronize(st);  // also before the ring has its next user
+    if (rc) return rc;
+    IMG2D_CUDA(err);
+    IMG2D_CUDA(done);
     return IMG2D_OK;
 }
 
@@ -1806,15 +1850,47 @@ static int run_dense(int ns, int nextrap, int nz, int nx, int nf, int nt, int M,
     if ((rc = sc.alloc(&dW, wel * sizeof(cpx)))) return rc;
     if ((rc = sc.alloc(&dS, wel * sizeof(cpx)))) return rc;
     if ((rc = sc.alloc(&dI, (size_t)ns * plane * sizeof(float)))) return rc;
-    if ((rc = upload(dF, opF, tab * sizeof(cpx), 0))) return rc;
-    if ((rc = upload(dB, opB, tab * sizeof(cpx), 0))) return rc;
-    if ((rc = upload(dW, wave, wel * sizeof(cpx), 0))) return rc;
-    if ((rc = upload(dS, shot, wel * sizeof(cpx), 0))) return rc;
-    MigrateArgs a = base_args(&plan, dW, dS);
-    a.denseF = dF;
-    a.denseB = dB;
-    if ((rc = launch(&plan, a, nullptr, dI, (long long)plane, 0))) return rc;
-    IMG2D_CUDA(cudaDeviceSynchronize());
+    IMG2D_CUDA(cudaMemcpy(dW, wave, wel * sizeof(cpx), cudaMemcpyHostToDevice));
+    IMG2D_CUDA(cudaMemcpy(dS, shot, wel * sizeof(cpx), cudaMemcpyHostToDevice));
+    // The tables go up in up to eight slabs of depth steps (16 MB or more each), on a stream of their
+    // own, while the kernel runs the slabs that have arrived (its wavefields pass from launch to launch
+    // through dW and dS).
+    const size_t depth = (size_t)nf * nx * L;  // table elements per depth step
+    const int slabs = std::max(1, std::min(nextrap, (int)std::min<size_t>(8, tab * sizeof(cpx) >> 24)));
+    auto first = [&](int c) { return (int)((long long)c * nextrap / slabs); };
+    std::vector<UploadPiece> pieces;
+    for (int c = 0; c < slabs; ++c) {
+        const size_t at = first(c) * depth, n = (first(c + 1) - first(c)) * depth;
+        add_pieces(pieces, dF + at, opF + at, n * sizeof(cpx), c);
+        add_pieces(pieces, dB + at, opB + at, n * sizeof(cpx), c);
+    }
+    struct Queue {
+        cudaStream_t s = nullptr;
+        cudaEvent_t e = nullptr;
+        ~Queue()
+        {
+            if (e) cudaEventDestroy(e);
+            if (s) cudaStreamDestroy(s);
+        }
+    } up;
+    IMG2D_CUDA(cudaStreamCreateWithFlags(&up.s, cudaStreamNonBlocking));
+    IMG2D_CUDA(cudaEventCreateWithFlags(&up.e, cudaEventDisableTiming));
+    IMG2D_CUDA(cudaMemset2DAsync(dI, plane * sizeof(float), 0, (size_t)nextrap * nx * sizeof(float), ns, 0));
+    rc = upload(pieces, slabs, up.s, [&](int c) -> int {
+        IMG2D_CUDA(cudaEventRecord(up.e, up.s));
+        IMG2D_CUDA(cudaStreamWaitEvent(0, up.e, 0));
+        MigrateArgs a = base_args(&plan, dW, dS);
+        a.nextrap = first(c + 1) - first(c);
+        a.denseF = dF + first(c) * depth;
+        a.denseB = dB + first(c) * depth;
+        a.image_shots = dI + (size_t)first(c) * nx;
+        a.img_sstride = (long long)plane;
+        IMG2D_CUDA(cudaMemsetAsync(plan.counter.p, 0, 2 * sizeof(int), 0));
+        return launch_kernel(&plan, a, plan.grid, 0);
+    });
+    const cudaError_t done = cudaDeviceSynchronize();  // nothing queued is left behind, errors or not
+    if (rc) return rc;
+    IMG2D_CUDA(done);
     // rows [0, nextrap) of every shot image
     IMG2D_CUDA(cudaMemcpy2D(image, plane * sizeof(float), dI, plane * sizeof(float),
                             (size_t)nextrap * nx * sizeof(float), ns, cudaMemcpyDeviceToHost));
