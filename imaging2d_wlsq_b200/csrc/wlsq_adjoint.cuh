@@ -206,7 +206,7 @@ __device__ __forceinline__ void fir_transposed_rt(const DemigrateArgs &a, const 
 #pragma unroll
     for (int jj = 0; jj < X; ++jj) {
         float r0 = 0.f, i0 = 0.f;
-        for (int k = 0; k < L; ++k) {
+        for (int k = L - 1; k >= 0; --k) {  // inputs in increasing position, as in fir_transposed
             const int xi = xb + jj + M - k;
             const float2 v = src[pad_slot(xi, X) * G + q];
             int xm = u0 + xi - Mp;

@@ -25,6 +25,7 @@
 #include "wlsq_adjoint.cuh"
 #include "wlsq_adjoint_cluster.cuh"
 #include "wlsq_rows_adjoint.cuh"
+#include "wlsq_adjoint_wide.cuh"
 #include "wlsq_frontend.cuh"
 
 namespace img2d {
@@ -200,29 +201,6 @@ struct DemigKernel {
 #define IMG2D_DEMIG(G, L) {G, L, demigrate_kernel<G, L, kAdjWarps>}
 #define IMG2D_DEMIG_G(G) IMG2D_DEMIG(G, 0), IMG2D_DEMIG(G, 25), IMG2D_DEMIG(G, 31), IMG2D_DEMIG(G, 35), IMG2D_DEMIG(G, 55)
 static const DemigKernel kDemig[] = {IMG2D_DEMIG_G(2), IMG2D_DEMIG_G(4), IMG2D_DEMIG_G(8)};
-
-struct DemigClusterKernel {
-    int L;
-    DemigFn fn;
-    DemigFn ring;  // forward steps through the shared-memory tap-pair ring (compile-time L only)
-};
-static const DemigClusterKernel kDemigCluster[] = {
-    {0, demigrate_cluster_kernel<0>, nullptr},
-    {25, demigrate_cluster_kernel<25>, demigrate_cluster_kernel<25, true>},
-    {31, demigrate_cluster_kernel<31>, demigrate_cluster_kernel<31, true>},
-    {35, demigrate_cluster_kernel<35>, demigrate_cluster_kernel<35, true>},
-    {55, demigrate_cluster_kernel<55>, demigrate_cluster_kernel<55, true>},
-};
-
-static DemigFn find_demig_cluster(int L, bool ring = false)
-{
-    DemigFn generic = nullptr;
-    for (const auto &k : kDemigCluster) {
-        if (k.L == L) return ring ? k.ring : k.fn;
-        if (k.L == 0) generic = k.fn;
-    }
-    return ring ? nullptr : generic;
-}
 
 // Row-split demigration kernels by slots per item and tap pairs per lane.
 struct DemigRowsKernel {
@@ -708,8 +686,9 @@ struct img2d_plan {
     // demigration (adjoint) launch state, built on its first call
     int adj_G = 0, adj_grid = 0, adj_items_n = 0, adj_wmax = 0, adj_block = 0, adj_slab = 0, adj_nslab = 0;
     int adj_cluster = 0;               // CTAs per cluster of the cluster demigration kernel, 0 = single CTA
-    bool adj_rows = false, adj_allow_rows = true;  // the row-split demigration kernel
+    bool adj_rows = false, adj_allow_rows = true, adj_allow_wide = true;  // the row-split demigration kernel
     void (*adj_rows_fn)(img2d::RowsAdjArgs) = nullptr;
+    void (*adj_wide_fn)(img2d::DemigrateArgs, int *) = nullptr;  // the wide demigration kernel
     bool adj_full_cache = false;       // kept source: every depth step of every item (else per-CTA planes only)
     bool adj_ring = false;             // its forward steps read operator pairs through the shared-memory ring
     bool model_set = false;            // set_model has built the padded tables and the operator index
@@ -1628,7 +1607,7 @@ static int demig_prepare(img2d_plan *p, int slab)
     if (slab <= 0) slab = 8;
     slab = std::min(slab, p->nextrap);
     const int nslab = (p->nextrap + slab - 1) / slab;
-    if ((p->adj_fn || p->adj_rows_fn) && p->adj_slab == slab) return IMG2D_OK;
+    if ((p->adj_fn || p->adj_rows_fn || p->adj_wide_fn) && p->adj_slab == slab) return IMG2D_OK;
     p->adj_cache_valid = false;  // the checkpoint layout depends on the slab depth
     int dev = 0, smem_optin = 0, nsm = 0;
     IMG2D_CUDA(cudaGetDevice(&dev));
@@ -1642,25 +1621,45 @@ static int demig_prepare(img2d_plan *p, int slab)
     bool ring = false;
     DemigFn fn = nullptr;
     size_t smem = 0;
-    // Cluster kernel (16 slots per item, 512 positions per CTA) when there are enough slots to fill
-    // it and the widest window fits 16 CTAs, with the forward steps' tap-pair ring where the operator
-    // length has an instance and its shared memory fits; otherwise the single-CTA kernel.
-    if (p->n_slots >= 12 && !(p->flags & IMG2D_FLAG_NO_CLUSTER)) {
+    // With enough slots to fill items of 16: the wide kernel (1024 positions per CTA; 7 to 65 taps), or the
+    // cluster kernel (512 positions, any length), where the widest window fits 16 CTAs; otherwise the
+    // row-split kernel or the single-CTA one.
+    void (*wide_fn)(DemigrateArgs, int *) = nullptr;
+    if (p->adj_allow_wide && p->n_slots >= 12 && !(p->flags & IMG2D_FLAG_NO_CLUSTER) && p->L >= 7 &&
+        demigw_smem_bytes(p->M) + static_reserve <= (size_t)smem_optin) {
+        widest = pack_groups(p, DemigWideShape::G, groups, segs, owner);
+        int k = (widest + DemigWideShape::PC - 1) / DemigWideShape::PC;
+        // operators of less than 17 taps need few pairs per step: the wait for the ring's first copies
+        // would be most of it
+        const bool wring = !(p->flags & IMG2D_FLAG_DEMIG_NO_RING) && p->L >= 17;
+        auto wf = wring ? demigrate_wide_kernel<true> : demigrate_wide_kernel<false>;
+        const size_t wsmem = demigw_smem_bytes(p->M);
+        // few items: windows are spread over more CTAs than they need, down to 256 positions each
+        auto fits = [&](int c) {
+            return c <= 8 || (c <= kMaxCluster && clusters_that_fit((const void *)wf, c, DemigWideShape::NW * 32, wsmem) > 0);
+        };
+        while ((long long)groups.size() * p->nf * k * 2 <= nsm && widest / (2 * k) >= 256 && fits(2 * k)) k *= 2;
+        if (fits(k)) {
+            K = k;
+            G = DemigWideShape::G;
+            wide_fn = wf;
+            smem = wsmem;
+            ring = wring;
+        }
+    }
+    if (!K && p->n_slots >= 12 && !(p->flags & IMG2D_FLAG_NO_CLUSTER)) {
         widest = pack_groups(p, 16, groups, segs, owner);
         const int k = (widest + kDcPC - 1) / kDcPC;
-        auto try_fn = [&](DemigFn cfn, size_t csmem, bool is_ring) {
-            if (!cfn || K || csmem + static_reserve > (size_t)smem_optin) return;
+        const DemigFn cfn = demigrate_cluster_kernel;
+        const size_t csmem = demigc_smem_bytes(p->M);
+        if (csmem + static_reserve <= (size_t)smem_optin) {
             if (k <= 8 || (k <= kMaxCluster && clusters_that_fit((const void *)cfn, k, kDcNW * 32, csmem) > 0)) {
                 K = k;
                 G = 16;
                 fn = cfn;
                 smem = csmem;
-                ring = is_ring;
             }
-        };
-        if (!(p->flags & IMG2D_FLAG_DEMIG_NO_RING))
-            try_fn(find_demig_cluster(p->L, true), demigc_ring_smem_bytes(p->M), true);
-        try_fn(find_demig_cluster(p->L), demigc_smem_bytes(p->M), false);
+        }
     }
     // Fewer slots: the row-split kernel, which keeps every S_l, where its shared memory fits.
     void (*rows_fn)(RowsAdjArgs) = nullptr;
@@ -1684,8 +1683,8 @@ static int demig_prepare(img2d_plan *p, int slab)
         fn = find_demig(G, p->L);
         smem = demig_smem_bytes(G, widest, p->M);
     }
-    if (!fn && !rows_fn) return fail(IMG2D_EINVAL, "no demigration kernel for this configuration");
-    const void *any_fn = rows_fn ? (const void *)rows_fn : (const void *)fn;
+    if (!fn && !rows_fn && !wide_fn) return fail(IMG2D_EINVAL, "no demigration kernel for this configuration");
+    const void *any_fn = rows_fn ? (const void *)rows_fn : (wide_fn ? (const void *)wide_fn : (const void *)fn);
     IMG2D_CUDA(cudaFuncSetAttribute(any_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     std::vector<int2> items;
     std::vector<int> gorder(groups.size());
@@ -1709,10 +1708,11 @@ static int demig_prepare(img2d_plan *p, int slab)
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int nclusters = 0;
-        IMG2D_CUDA(cudaOccupancyMaxActiveClusters(&nclusters, (void *)fn, &cfg));
+        IMG2D_CUDA(cudaOccupancyMaxActiveClusters(&nclusters, (void *)any_fn, &cfg));
         if (nclusters <= 0) return fail(IMG2D_ECUDA, "no demigration cluster of this size fits on the device");
         grid = (int)std::min<size_t>(items.size(), (size_t)nclusters) * K;
-        const long long pe4 = (long long)kDcPC * kDcQ;  // float4 per plane
+        // float4 per plane
+        const long long pe4 = wide_fn ? (long long)DemigWideShape::PC * DemigWideShape::ROW : (long long)kDcPC * kDcQ;
         work_cta = 2 * (long long)(nslab + slab + 1) * pe4;
         cache_item = 2 * (long long)K * nslab * pe4;
     } else if (rows_fn) {
@@ -1755,7 +1755,11 @@ static int demig_prepare(img2d_plan *p, int slab)
     if ((rc = p->adj_segs.ensure(segs.size() * sizeof(int4)))) return rc;
     if ((rc = p->adj_owner.ensure(owner.size() * sizeof(int16_t)))) return rc;
     if ((rc = p->adj_counter.ensure(sizeof(int)))) return rc;
-    if (!rows_fn && (rc = p->adj_work.ensure((size_t)grid * work_cta * sizeof(float2)))) return rc;
+    if (!rows_fn && (rc = p->adj_work.ensure((size_t)grid * work_cta * sizeof(float2)))) {
+        if (rc != IMG2D_ENOMEM || !wide_fn) return rc;
+        p->adj_allow_wide = false;  // the cluster kernel's planes are half as large
+        return demig_prepare(p, slab);
+    }
     IMG2D_CUDA(cudaMemcpy(p->adj_items.p, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice));
     IMG2D_CUDA(cudaMemcpy(p->adj_groups.p, groups.data(), groups.size() * sizeof(GroupDesc), cudaMemcpyHostToDevice));
     IMG2D_CUDA(cudaMemcpy(p->adj_segs.p, segs.data(), segs.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -1766,6 +1770,7 @@ static int demig_prepare(img2d_plan *p, int slab)
     p->adj_wmax = widest;
     p->adj_block = K ? kDcNW * 32 : block;
     p->adj_rows = rows_fn != nullptr;
+    p->adj_wide_fn = wide_fn;
     p->adj_rows_fn = rows_fn;
     p->adj_full_cache = rows_fn && (long long)items.size() * cache_item <= kDemigRowsCacheElems;
     p->adj_cluster = K;
@@ -2223,7 +2228,15 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
         cfg.stream = st;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_fn, a));
+        if (p->adj_wide_fn) {
+            // its bounded waits report to the plan's status word
+            int *status = p->counter.as<int>() + 1;
+            IMG2D_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
+            p->launched = true;
+            IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_wide_fn, a, status));
+        } else {
+            IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_fn, a));
+        }
     } else if (p->adj_rows) {
         if (!p->rows_tab_set && (rc = set_rows_table(p, st))) return rc;
         RowsAdjArgs ra{};
@@ -2251,7 +2264,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
 int img2d_plan_describe_demigration(const img2d_plan *p, char *buf, int buflen)
 {
     if (!p || !buf || buflen <= 0) return fail(IMG2D_EINVAL, "bad describe arguments");
-    if (!p->adj_fn && !p->adj_rows_fn) return fail(IMG2D_EINVAL, "no demigration has run on this plan yet");
+    if (!p->adj_fn && !p->adj_rows_fn && !p->adj_wide_fn) return fail(IMG2D_EINVAL, "no demigration has run on this plan yet");
     snprintf(buf, buflen,
              "{\"kernel\": \"%s\", \"cluster\": %d, \"G\": %d, \"X\": 8, \"L\": %d, \"grid\": %d, \"block\": %d, "
              "\"smem\": %zu, \"items\": %d, \"max_union_width\": %d, \"slab\": %d, \"slabs\": %d, "
