@@ -233,6 +233,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
             const int xm = min(u0 + x, a.nx - 1);
             off0[x] = (unsigned)idx_j[xm] * (unsigned)ROWB;
             off1[x] = a.nextrap > 1 ? (unsigned)idx_j[a.idx_lstride + xm] * (unsigned)ROWB : 0u;
+            off2[x] = 0u;  // with two steps the last one looks ahead to it
         }
         for (int i = threadIdx.x; i < G * (wp / X); i += T) {
             const int g = i / (wp / X), b = i % (wp / X);

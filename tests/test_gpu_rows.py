@@ -146,3 +146,13 @@ def test_rows_demigration_with_little_memory_takes_the_slab_kernel():
     assert op.plan.describe_demigration()["kernel"] == "demigrate"
     assert rel_l2(d.cpu().numpy(), ref) <= 1e-5
     op.plan.close()
+
+
+@pytest.mark.parametrize("ns", [1, 2])
+@pytest.mark.parametrize("nz", [1, 2, 3])
+def test_rows_few_depth_steps(ns, nz):
+    """The last depth step looks ahead to row offsets of a step that does not exist."""
+    w = _survey(ns, 300, nz, 4, 7)
+    assert _kernel(w)["kernel"] == "migrate_rows"
+    img, _, wave, shot = migration.migrate_workload(w)
+    _check(w, img, wave, shot)
