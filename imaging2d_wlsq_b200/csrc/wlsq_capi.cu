@@ -82,24 +82,23 @@ static KernelFn find_fixed(int G, int L)
     return nullptr;
 }
 
-// Row-split kernels by slots per item, tap pairs per lane and number of tables; 4 outputs per quad.
-// One slot keeps its rows' next taps in registers (the row loads are its whole traffic: 3.36 against
-// 3.76 ms for one shot of 1024 x 500, 256 frequencies, 31 taps); with two slots those registers are
-// better left to the second slot (32 shots, two tables: 3.2 against 4.2 ms with one slot an item).
-// Tried on the same cases and slower: 8 outputs per quad with one slot (3.58 ms, 168 registers, and
-// 3.45 without the held taps), three CTAs per SM at 80 registers (3.76), 4 slots per item (spills).
+// Row-split kernels by slots per item, tap pairs per lane and number of tables; 4 outputs per quad, a
+// row's next taps held in registers.  Tried on one shot of 1024 x 500, 256 frequencies, 31 taps (3.36
+// ms) and slower: 8 outputs per quad (3.58 ms, 168 registers; 3.45 without the held taps), three CTAs
+// per SM at 80 registers (3.76), 4 slots per item (spills).  With two slots packed multiply-adds and
+// held taps together gave 3 to 6% (9 shots, two tables: 643 -> 603 us), neither alone did.
 struct RowsKernel {
     int G, np;
     bool two;
     KernelFn fn;
 };
-#define IMG2D_ROWS(G, NP, PIPE) \
-    {G, NP, false, migrate_rows_kernel<G, NP, false, PIPE>}, {G, NP, true, migrate_rows_kernel<G, NP, true, PIPE>}
-#define IMG2D_ROWS_NP(G, PIPE)                                                                            \
-    IMG2D_ROWS(G, 1, PIPE), IMG2D_ROWS(G, 2, PIPE), IMG2D_ROWS(G, 3, PIPE), IMG2D_ROWS(G, 4, PIPE),       \
-        IMG2D_ROWS(G, 5, PIPE), IMG2D_ROWS(G, 6, PIPE), IMG2D_ROWS(G, 7, PIPE), IMG2D_ROWS(G, 8, PIPE),   \
-        IMG2D_ROWS(G, 10, PIPE)
-static const RowsKernel kRows[] = {IMG2D_ROWS_NP(1, true), IMG2D_ROWS_NP(2, false)};
+#define IMG2D_ROWS(NP)                                                                         \
+    {1, NP, false, migrate_rows_kernel<1, NP, false>}, {1, NP, true, migrate_rows_kernel<1, NP, true>},  \
+        {2, NP, false, migrate_rows_kernel<2, NP, false>}, {2, NP, true, migrate_rows_kernel<2, NP, true>}
+static const RowsKernel kRows[] = {
+    IMG2D_ROWS(1), IMG2D_ROWS(2), IMG2D_ROWS(3), IMG2D_ROWS(4), IMG2D_ROWS(5),
+    IMG2D_ROWS(6), IMG2D_ROWS(7), IMG2D_ROWS(8), IMG2D_ROWS(10),
+};
 
 static KernelFn find_rows(int G, int L, bool two)
 {
@@ -1217,14 +1216,20 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             if (mode == OP_TWO || p->n_slots < 6) {
                 p->rows = true;
             } else {
-                // wide kernel: 8 slots x up to 1024 positions per CTA; cluster2: 16 x 512
+                // Time of a depth step of the wide kernel (8 slots x up to 1024 positions per CTA) or of the
+                // 16-slot one (up to 512), in microseconds, for a CTA with all warps busy: fitted on a
+                // B200 to 25 to 55 taps, windows of 256 to 1024 positions.  Clusters of three and more
+                // leave about 9% of the SMs idle.  The row-split estimate is 8% low on average (16
+                // surveys of 7 to 179 shots).
                 const bool wide = want_wide;
                 const int G = wide ? WideShape::G : 16, pc = wide ? WideShape::PC : 512;
                 const int widest = make_groups(G), K = (widest + pc - 1) / pc;
-                const int nc = wide ? std::min(pc, (widest + K * 256 - 1) / (K * 256) * 256) : pc;
-                const double item = (wide ? wide_item_cost(nc, 1) * 17.0 : 17.0) * (p->L + 5) / 40.0;
-                const double waves = (double)groups.size() * nf * K / nsm;
-                p->rows = rows_l.us < 0.95 * item * (waves <= 4.0 ? std::ceil(waves) : waves + 0.5);
+                const int nc = std::min(pc, (widest + K * 256 - 1) / (K * 256) * 256);
+                const double item = wide ? 0.344 * (p->L + 15) * wide_item_cost(nc, 1)
+                                         : 0.375 * (p->L + 7.4) * (nc == pc ? 1.0 : 0.57);
+                const int clusters = std::max(1, (K > 2 ? nsm * 91 / 100 : nsm) / K);
+                const double waves = (double)groups.size() * nf / clusters;
+                p->rows = 1.08 * rows_l.us < item * (waves <= 4.0 ? std::ceil(waves) : waves + 0.5);
             }
         }
     }

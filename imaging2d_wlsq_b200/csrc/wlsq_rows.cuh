@@ -12,15 +12,16 @@
 //
 // Measured on a B200 (whole call, against the single-CTA kernels before): one shot of 1024 x 500 with
 // 256 frequencies and 31 taps 10.7 -> 3.72 ms (17.6 TFLOP/s), 4 shots of 320 x 200, 64 frequencies,
-// 25 taps 0.97 -> 0.50 ms, 9 shots of 151 x 136, 60 frequencies, 43 taps and two tables 3.50 -> 0.68 ms.
+// 25 taps 0.97 -> 0.44 ms, 9 shots of 151 x 136, 60 frequencies, 43 taps and two tables 3.50 -> 0.63 ms.
 // In the one-shot case L1 serves 68% of the row sectors and its data pipe is 54% busy, issue slots 51%;
 // with 12 to 16 warps of 128 registers per SM neither fills up.
 //
 // Wavefields of an item (G slots x one frequency) stay in shared memory, two buffers in turn, one
-// barrier per depth step.  A position is one float4 (S.re, S.im, R.re, R.im), R conjugated in the
-// single-table mode; one unused float4 after every 8 positions spreads a quad's four tap ranges over
-// the banks.  The operator row offsets come from shared memory, where each step stores those of the
-// step after next.
+// barrier per depth step.  A position is one float4 (S.re, S.im, R.re, R.im) with one slot, and with
+// two slots a, b one float4 of S (a.re, b.re, a.im, b.im) and one of R, so that the multiply-adds are
+// packed (FFMA2); R is conjugated in the single-table mode.  One unused float4 after every 8 positions
+// spreads a quad's four tap ranges over the banks.  The operator row offsets come from shared memory,
+// where each step stores those of the step after next.
 //
 // Image: the first item of a CTA stores its rows of the CTA's partial image (nothing has to be zeroed
 // or read), later ones add with Kahan compensation; the reduction reads what the CTA's item count
@@ -145,9 +146,9 @@ __device__ __forceinline__ void rows_load8(RowTaps &t, const char *p)
         : "l"(p));
 }
 
-// G: lane slots per item.  NP: tap pairs per lane.  PIPE: a row's next taps are held in registers.  TWO: forward and backward
+// G: lane slots per item.  NP: tap pairs per lane.  TWO: forward and backward
 // table; else the receiver uses the conjugated forward rows.
-template <int G, int NP, bool TWO, bool PIPE>
+template <int G, int NP, bool TWO>
 __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateArgs a)
 {
     constexpr int X = kRowsX, Q = 2 * NP;
@@ -251,7 +252,16 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
             const cpx *rs = a.shot + a.shot_off[sg.x] + (long long)j * sg.w;
             for (int i = threadIdx.x; i < sg.w; i += T) {
                 const cpx S = ws[i], V = rs[i];
-                bufA[(size_t)sg.y * ns + rows_pad(left + sg.z - u0 + i)] = make_float4(S.re, S.im, V.re, TWO ? V.im : -V.im);
+                const int at = rows_pad(left + sg.z - u0 + i);
+                if (G == 2) {
+                    float *fs = reinterpret_cast<float *>(bufA + at) + sg.y, *fr = reinterpret_cast<float *>(bufA + ns + at) + sg.y;
+                    fs[0] = S.re;
+                    fs[2] = S.im;
+                    fr[0] = V.re;
+                    fr[2] = TWO ? V.im : -V.im;
+                } else {
+                    bufA[at] = make_float4(S.re, S.im, V.re, TWO ? V.im : -V.im);
+                }
             }
         }
         // The taps of a row's first chunk are always loaded one block ahead (across the step boundary
@@ -259,7 +269,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
         // are refilled as soon as they have been read.
         unsigned off[X];
         Taps tp[X];
-        if (PIPE && warp < nwb) {
+        if (warp < nwb) {
             load_off(off, off0 + (warp * 8 + p) * X);
 #pragma unroll
             for (int jj = 0; jj < X; ++jj) load_taps(tp[jj], off[jj], 0);
@@ -296,7 +306,6 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
                         pc[i] = x < W && done > 1 ? crow[u0 + x] : 0.f;
                     }
                 }
-                if (!PIPE) load_off(off, off0 + xb);
                 float acc[X][G][4];
                 // inputs i = 0 ... Q + X - 2 of this lane, from position left + xb - M + tap0: that is
                 // 8-row hi, element e + i, one pad entry further after each row end
@@ -315,7 +324,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         if (i < nt) load_in(4 * c + X - 1 + i, win[X - 1 + i]);
-                    if (PIPE && c == NF - 1) {
+                    if (c == NF - 1) {
                         // row offsets of this warp's next block: of this step, or the first of the next
                         const unsigned *os = wb + nwarps < nwb ? off0 + xb + nwarps * WP_POS
                                                                : off1 + (warp * 8 + p) * X;
@@ -328,6 +337,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
                         for (int g = 0; g < G; ++g) {
                             const float4 v = win[jj + d][g];
                             float (&s)[4] = acc[jj][g];
+                            if (G == 2) {
+                                // both slots' S (g = 0) or R (g = 1) at once
+                                const float tr = g ? br : fr, ti = g ? bi : fi;
+                                float2 *s2 = reinterpret_cast<float2 *>(s);
+                                const float2 re = make_float2(v.x, v.y), im = make_float2(v.z, v.w);
+                                if (c == 0 && d == 0) {
+                                    s2[0] = make_float2(tr * v.x, tr * v.y);
+                                    s2[1] = make_float2(tr * v.z, tr * v.w);
+                                } else {
+                                    s2[0] = __ffma2_rn(make_float2(tr, tr), re, s2[0]);
+                                    s2[1] = __ffma2_rn(make_float2(tr, tr), im, s2[1]);
+                                }
+                                s2[0] = __ffma2_rn(make_float2(-ti, -ti), im, s2[0]);
+                                s2[1] = __ffma2_rn(make_float2(ti, ti), re, s2[1]);
+                                continue;
+                            }
                             if (c == 0 && d == 0) {
                                 s[0] = fr * v.x; s[1] = fr * v.y; s[2] = br * v.z; s[3] = br * v.w;
                             } else {
@@ -340,21 +365,18 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
                     };
 #pragma unroll
                     for (int jj = 0; jj < X; ++jj) {
-                        if (!PIPE) load_taps(tp[jj], off[jj], c);
 #pragma unroll
                         for (int d = 0; d < 4; ++d)
                             if (d < nt && (c < NF - 1 || d < nt - 1)) tap(jj, d);
-                        if (PIPE && c < NF - 1) load_taps(tp[jj], off[jj], c + 1);
+                        if (c < NF - 1) load_taps(tp[jj], off[jj], c + 1);
                     }
                     if (c == NF - 1) {
                         if (last_tap) {
 #pragma unroll
                             for (int jj = 0; jj < X; ++jj) tap(jj, nt - 1);
                         }
-                        if (PIPE) {
 #pragma unroll
-                            for (int jj = 0; jj < X; ++jj) load_taps(tp[jj], off[jj], 0);
-                        }
+                        for (int jj = 0; jj < X; ++jj) load_taps(tp[jj], off[jj], 0);
                     }
 #pragma unroll
                     for (int i = 0; i < X - 1; ++i)
@@ -366,41 +388,41 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
                 float img[R];
 #pragma unroll
                 for (int i = 0; i < R; ++i) img[i] = 0.f;
+                static_assert(R == 1, "a lane keeps one of the quad's four outputs");
+                float out[G][4];
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    const unsigned m = mask[g * (wp / X) + b] >> (r * R);
-                    float out[R][4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        float h[X / 2];
+                        float h[2];
 #pragma unroll
-                        for (int i = 0; i < X / 2; ++i) {
-                            const float keep = hi2 ? acc[X / 2 + i][g][e] : acc[i][g][e];
-                            const float send = hi2 ? acc[i][g][e] : acc[X / 2 + i][g][e];
+                        for (int i = 0; i < 2; ++i) {
+                            const float keep = hi2 ? acc[2 + i][g][e] : acc[i][g][e];
+                            const float send = hi2 ? acc[i][g][e] : acc[2 + i][g][e];
                             h[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
                         }
-#pragma unroll
-                        for (int i = 0; i < R; ++i) {
-                            const float keep = hi1 ? h[R + i] : h[i];
-                            const float send = hi1 ? h[i] : h[R + i];
-                            out[i][e] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < R; ++i) {
-                        const bool in = (m >> i) & 1u;
-                        const float sr = in ? out[i][0] : 0.f, si = in ? out[i][1] : 0.f;
-                        const float rr = in ? out[i][2] : 0.f, ri = in ? out[i][3] : 0.f;
-                        const int x = xb + r * R + i;
-                        bufB[(size_t)g * ns + rows_pad(left + x)] = make_float4(sr, si, rr, ri);
-                        const float v = TWO ? sr * rr + si * ri : sr * rr - si * ri;
-                        img[i] += v;
-                        if (a.image_shots && in) {
-                            const int s = a.owner[grp.owner_off + (long long)g * grp.owner_stride + x];
-                            atomicAdd(a.image_shots + (long long)s * a.img_sstride + (long long)l * a.nx + u0 + x, v);
-                        }
+                        const float keep = hi1 ? h[1] : h[0], send = hi1 ? h[0] : h[1];
+                        out[g][e] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
                     }
                 }
+                const int xo = xb + r;  // this lane's output
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    // slot g: its components among out[]
+                    float &sr = G == 2 ? out[0][g] : out[g][0], &si = G == 2 ? out[0][2 + g] : out[g][1];
+                    float &rr = G == 2 ? out[G - 1][g] : out[g][2], &ri = G == 2 ? out[G - 1][2 + g] : out[g][3];
+                    const bool in = (mask[g * (wp / X) + b] >> r) & 1u;
+                    if (!in) sr = si = rr = ri = 0.f;
+                    const float v = TWO ? sr * rr + si * ri : sr * rr - si * ri;
+                    img[0] += v;
+                    if (a.image_shots && in) {
+                        const int s = a.owner[grp.owner_off + (long long)g * grp.owner_stride + xo];
+                        atomicAdd(a.image_shots + (long long)s * a.img_sstride + (long long)l * a.nx + u0 + xo, v);
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < G; ++g)
+                    bufB[(size_t)g * ns + rows_pad(left + xo)] = make_float4(out[g][0], out[g][1], out[g][2], out[g][3]);
                 if (more) {
 #pragma unroll
                     for (int i = 0; i < R; ++i) off2[xb + r * R + i] = nidx[i] * (unsigned)ROWB;
@@ -436,9 +458,17 @@ __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateAr
                 cpx *ws = a.wave + a.shot_off[sg.x] + (long long)j * sg.w;
                 cpx *rs = a.shot + a.shot_off[sg.x] + (long long)j * sg.w;
                 for (int i = threadIdx.x; i < sg.w; i += T) {
-                    const float4 v = bufA[(size_t)sg.y * ns + rows_pad(left + sg.z - u0 + i)];
-                    ws[i] = cpx{v.x, v.y};
-                    rs[i] = cpx{v.z, TWO ? v.w : -v.w};
+                    const int at = rows_pad(left + sg.z - u0 + i);
+                    if (G == 2) {
+                        const float *fs = reinterpret_cast<const float *>(bufA + at) + sg.y;
+                        const float *fr = reinterpret_cast<const float *>(bufA + ns + at) + sg.y;
+                        ws[i] = cpx{fs[0], fs[2]};
+                        rs[i] = cpx{fr[0], TWO ? fr[2] : -fr[2]};
+                    } else {
+                        const float4 v = bufA[at];
+                        ws[i] = cpx{v.x, v.y};
+                        rs[i] = cpx{v.z, TWO ? v.w : -v.w};
+                    }
                 }
             }
         }
