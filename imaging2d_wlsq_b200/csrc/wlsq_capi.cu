@@ -473,8 +473,8 @@ static void device_free(void *p, size_t n, int dev)
 
 // Pinned staging for uploads from pageable memory.  A plain cudaMemcpy of pageable memory runs at the
 // speed of one host thread (about 10 GB/s here); four workers copying 2 MB pieces into a pinned ring,
-// each sending its own, reach 34 GB/s (eight 31, sixteen 22).  One upload uses the ring at a time, others take the plain
-// copy.  The ring (16 MB) is kept until img2d_release_host_cache.
+// each sending its own, reach 34 GB/s (eight 31, sixteen 22).  One upload uses the ring at a time,
+// others take the plain copy.  The ring (16 MB) is kept until img2d_release_host_cache.
 constexpr size_t kStagePiece = 2 << 20;
 constexpr int kStageWorkers = 4;
 struct StageRing {

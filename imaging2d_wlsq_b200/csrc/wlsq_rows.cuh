@@ -11,8 +11,8 @@
 // the same rows (k = w/v changes slowly with depth), and L1 keeps what shared memory leaves free.
 //
 // Measured on a B200 (whole call, against the single-CTA kernels before): one shot of 1024 x 500 with
-// 256 frequencies and 31 taps 10.7 -> 3.72 ms (17.6 TFLOP/s), 4 shots of 320 x 200, 64 frequencies,
-// 25 taps 0.97 -> 0.44 ms, 9 shots of 151 x 136, 60 frequencies, 43 taps and two tables 3.50 -> 0.63 ms.
+// 256 frequencies and 31 taps 10.7 -> 3.8 ms (17 TFLOP/s), 4 shots of 320 x 200, 64 frequencies,
+// 25 taps 0.97 -> 0.45 ms, 9 shots of 151 x 136, 60 frequencies, 43 taps and two tables 3.50 -> 0.63 ms.
 // In the one-shot case L1 serves 68% of the row sectors and its data pipe is 54% busy, issue slots 51%;
 // with 12 to 16 warps of 128 registers per SM neither fills up.
 //
@@ -146,8 +146,8 @@ __device__ __forceinline__ void rows_load8(RowTaps &t, const char *p)
         : "l"(p));
 }
 
-// G: lane slots per item.  NP: tap pairs per lane.  TWO: forward and backward
-// table; else the receiver uses the conjugated forward rows.
+// G: lane slots per item.  NP: tap pairs per lane.  TWO: forward and backward table; else the receiver
+// uses the conjugated forward rows.
 template <int G, int NP, bool TWO>
 __global__ void __launch_bounds__(kRowsThreads, 1) migrate_rows_kernel(MigrateArgs a)
 {

@@ -114,8 +114,9 @@ int img2d_migrate_compact(int ns, int nextrap, int nz, int nx, int nf, int nt, i
                           img2d_c64 *shot_fs, float *image, float *image_shots, int flags);
 /* img2d_migrate_compact keeps, per device, its plan (for the last geometry on that device) and its
  * device buffers (grown to the largest sizes seen) between calls, so repeated calls allocate
- * nothing.  img2d_release_host_cache frees them on every device; img2d_host_cache_device_count
- * is the number of devices that hold such a cache.
+ * nothing.  img2d_release_host_cache frees them on every device, with the pinned buffers of the
+ * uploads and the released device blocks that are kept for the next plan or dense call;
+ * img2d_host_cache_device_count is the number of devices that hold a plan cache.
  * With 64 MiB of wavefields or more (and no per-shot images) a call runs in 8 frequency chunks: the
  * host copies of each chunk overlap the kernels of the others (pinned host memory overlaps fully),
  * on streams of its own, with a second set of per-CTA image partials.  It returns when everything
@@ -159,8 +160,8 @@ void img2d_plan_destroy(img2d_plan *plan);
 int img2d_plan_kernel_ms(img2d_plan *plan, float *ms);
 
 /* Status of the last migration launch on this plan, read on `stream` after it (waits for it):
- * IMG2D_ECUDA if a bounded wait inside the kernel gave up (the bulk-copy ring of
- * IMG2D_FLAG_WIDE_BULK; the results of that launch are then invalid), else IMG2D_OK.
+ * IMG2D_ECUDA if a bounded wait inside the kernel gave up (the wide migration and demigration
+ * kernels; the results of that launch are then invalid), else IMG2D_OK.
  * img2d_migrate_compact checks it by itself. */
 int img2d_plan_status(img2d_plan *plan, void *stream);
 
