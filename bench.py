@@ -40,8 +40,8 @@ UNIT = "pts/s"
 # dram = (dram__bytes_read.sum + dram__bytes_write.sum) / points, l2 = lts__t_sectors.sum * 32 / points.
 # Keyed by (kernel, variant) of describe(); the bench scales them by the points of its launch.
 TRAFFIC_PER_POINT = {
-    ("migrate_wide", 3): {"dram": 2.38, "l2": 82.4,
-                          "capture": "migrate_wide_kernel<1, 1, 0>, window packing, nz=60 nf=64"},
+    ("migrate_wide", 3): {"dram": 2.43, "l2": 69.5,
+                          "capture": "migrate_wide_kernel<1, 1, 0, 4, 1>, window packing, nz=60 nf=64"},
     ("migrate_cluster2", 11): {"dram": 0.980, "l2": 45.8, "capture": "migrate_cluster2_kernel ring variant, nz=60 nf=64"},
 }
 
@@ -426,7 +426,7 @@ def frontend_leg(dev, w):
         "records": {"value": samples / t_rec, "unit": "time samples/s", "ms": t_rec * 1e3,
                     "hbm_gbs": (4.0 * ns * nt * nx + 8.0 * 2 * ns * (nt // 2 + 1) * nx + 8.0 * nf * w.shot_nx.sum())
                                / t_rec / 1e9,
-                    "kernel": "cuFFT real-to-complex along time + pack_spectra_kernel (first nf rows, apertures)"},
+                    "kernel": "record_spectra_kernel (cuFFT + pack_spectra_kernel for lengths without a usable factor)"},
         "sources": {"value": ns * nt * nx / t_src, "unit": "time samples/s", "ms": t_src * 1e3},
         "cpu_reference_fft": {"value": nt * nx / c_fft, "unit": "time samples/s", "ms_per_shot": c_fft * 1e3,
                               "cores": 1, "kind": "reference",
