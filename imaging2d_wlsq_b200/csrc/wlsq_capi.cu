@@ -2491,10 +2491,10 @@ static std::map<int, FrontScratch> g_front;
 // multiply-adds per trace; none (N1 = 0) where that exceeds 150 nt (a prime nt: cuFFT is taken) or the
 // inner sums of 8 traces do not fit in shared memory.  16 traces per CTA (64-byte reads) unless only 8
 // leave room for two CTAs per SM.
-static SpecPlan spec_plan(int nt, int nf, size_t smem_optin)
+static SpecPlan spec_plan(int nt, int nf, size_t smem_optin, double &best_cost)
 {
     SpecPlan best{};
-    double best_cost = 150.0 * nt;
+    best_cost = 150.0 * nt;
     for (int N1 = 1; N1 <= 31 && N1 <= nt; ++N1) {
         if (nt % N1) continue;
       for (int M : {8, 10}) {
@@ -2609,8 +2609,15 @@ int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const 
     IMG2D_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     std::lock_guard<std::mutex> lock(g_front_mu);
     FrontScratch &fs = g_front[dev];
-    const SpecPlan pl = spec_plan(nt, nf, (size_t)smem_optin);
-    if (!pl.N1) return spectra_by_cufft(fs, ns, nt, nx, nf, d_records, x0, w, off, (cpx *)d_out, st);
+    double cost;
+    const SpecPlan pl = spec_plan(nt, nf, (size_t)smem_optin, cost);
+    // cuFFT transforms all nx traces to all rows: about 0.5 ms of launches and 8.5 ps per sample.  It
+    // is the faster one where most rows of many full-width records are kept (256 x 1024 x 2048 samples
+    // to 512 rows: 6.0 ms here, 5.0 ms with cuFFT; 32 x 1024 x 1024 to 512 rows: 0.43 and 1.0 ms).
+    double traces = 0.0;
+    for (int x : w) traces += x;
+    const bool library = 8.2e-11 * cost * traces > 0.5 + 8.5e-9 * ns * nt * (double)nx;
+    if (!pl.N1 || library) return spectra_by_cufft(fs, ns, nt, nx, nf, d_records, x0, w, off, (cpx *)d_out, st);
     const size_t n1 = (size_t)kSpecK * kSpecK, n2 = (size_t)pl.N2 * pl.mp, n3 = (size_t)nt;
     if ((rc = fs.tables.ensure((n1 + n2 + n3) * sizeof(float2)))) return rc;
     float2 *T1 = fs.tables.as<float2>(), *B = T1 + n1, *A = B + n2;

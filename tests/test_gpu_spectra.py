@@ -44,3 +44,14 @@ def test_source_spectra_match_transform_of_the_wavelets(nt, nf, dt, fpeak):
     ref = np.fft.fft((1.0 - 2.0 * term) * np.exp(-term) / np.sqrt(r)[:, None, :], axis=1)[:, :nf]
     assert rel_l2(got[:, :nf], ref) <= 2e-6
     assert np.all(got[:, nf:] == 0)
+
+
+def test_record_spectra_of_many_full_width_records():
+    """A call large enough for the library transform, checked on its first and last record."""
+    import torch
+    ns, nt, nx, nf = 128, 1024, 2048, 512
+    rec = torch.randn((ns, nt, nx), generator=torch.Generator("cuda").manual_seed(5), device="cuda")
+    got = frontend.records_to_spectra(rec, nf).reshape(ns, nf, nx)
+    for s in (0, ns - 1):
+        ref = np.fft.fft(rec[s].cpu().numpy().astype(np.float64), axis=0)[:nf]
+        assert rel_l2(got[s].cpu().numpy(), ref) <= 2e-6
