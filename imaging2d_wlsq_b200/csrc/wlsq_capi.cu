@@ -2560,9 +2560,11 @@ static int spectra_by_cufft(FrontScratch &fs, int ns, int nt, int nx, int nf, co
     }
     const cufftHandle plan = itp->second;
     if (cufftSetStream(plan, st) != CUFFT_SUCCESS) return fail(IMG2D_ECUDA, "cufftSetStream failed");
-    // cuFFT reads 8-byte pairs: with an odd nt * nx every other shot goes through an aligned copy
-    const bool odd = ns > 1 && ((long long)nt * nx & 1);
-    if ((rc = fs.spec.ensure((size_t)group * shot_spec * sizeof(cpx) + (odd ? (size_t)nt * nx * sizeof(float) : 0)))) return rc;
+    // cuFFT reads 8-byte pairs: a shot whose records start between two goes through an aligned copy (with
+    // an odd nt * nx every other one; all of them or the others where the caller's array itself does)
+    auto between = [&](int s) { return (reinterpret_cast<uintptr_t>(d_records + (long long)s * nt * nx) & 7) != 0; };
+    const bool copies = between(0) || (ns > 1 && between(1));
+    if ((rc = fs.spec.ensure((size_t)group * shot_spec * sizeof(cpx) + (copies ? (size_t)nt * nx * sizeof(float) : 0)))) return rc;
     cpx *d_spec = fs.spec.as<cpx>();
     float *aligned = reinterpret_cast<float *>(d_spec + (long long)group * shot_spec);
     Scratch sc;
@@ -2578,7 +2580,7 @@ static int spectra_by_cufft(FrontScratch &fs, int ns, int nt, int nx, int nf, co
         const int nsc = std::min(group, ns - s0);
         for (int k = 0; k < nsc; ++k) {
             cufftReal *in = const_cast<cufftReal *>(d_records + (long long)(s0 + k) * nt * nx);
-            if (odd && ((s0 + k) & 1)) {
+            if (between(s0 + k)) {
                 IMG2D_CUDA(cudaMemcpyAsync(aligned, in, (size_t)nt * nx * sizeof(float), cudaMemcpyDeviceToDevice, st));
                 in = aligned;
             }
