@@ -1551,18 +1551,26 @@ static int launch(img2d_plan *p, MigrateArgs a, float *d_image, float *d_image_s
     return IMG2D_OK;
 }
 
-// The row-split kernels' copy of the plan's tables.
+// The row-split kernels' copy of the plan's tables.  Made by set_model where migration uses it, and by the
+// first demigration that does; from then on every set_model renews it, so that a captured call,
+// which holds the address and not the copying, reads the model of the last set_model.
+static size_t rows_table_bytes(const img2d_plan *p)
+{
+    return (size_t)p->nk * rows_row_floats(p->L, p->mode == OP_TWO) * sizeof(float);
+}
 static int set_rows_table(img2d_plan *p, cudaStream_t st)
 {
     const bool two = p->mode == OP_TWO;
-    const long long floats = (long long)p->nk * rows_row_floats(p->L, two);
-    const int rc = p->tab_rows.ensure((size_t)floats * sizeof(float));
+    const long long floats = (long long)(rows_table_bytes(p) / sizeof(float));
+    const int rc = p->tab_rows.ensure(rows_table_bytes(p));
     if (rc) return rc;
     rows_table_kernel<<<(int)std::min<long long>((floats / 2 + 255) / 256, 148 * 8), 256, 0, st>>>(
         p->tabF.as<cpx>(), two ? p->tabB.as<cpx>() : nullptr, p->tab_stride, p->L, rows_np(p->L), rows_starts(p->L),
         p->nk, p->tab_rows.as<float>());
     IMG2D_CUDA(cudaGetLastError());
-    p->rows_tab_set = true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture == cudaStreamCaptureStatusNone) p->rows_tab_set = true;  // a captured copy has not run yet
     return IMG2D_OK;
 }
 
@@ -1580,8 +1588,7 @@ static int set_model(img2d_plan *p, const double *d_omega, const double *d_vel, 
         IMG2D_CUDA(cudaMemsetAsync(p->tabB.p, 0, (size_t)p->nk * prow, st));
         IMG2D_CUDA(cudaMemcpy2DAsync(p->tabB.p, prow, d_tabB, row, row, p->nk, cudaMemcpyDeviceToDevice, st));
     }
-    p->rows_tab_set = false;
-    if (p->rows) {
+    if (p->rows || p->tab_rows.p) {
         const int rc = set_rows_table(p, st);
         if (rc) return rc;
     }
@@ -2172,6 +2179,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
             rc = p->adj_cache.ensure(p->adj_full_cache ? (size_t)p->adj_items_n * p->adj_cache_item * sizeof(float2) : 16);
         if (!rc && !(p->adj_full_cache && source_mode != IMG2D_SOURCE_RECOMPUTE))
             rc = p->adj_work.ensure((size_t)p->adj_grid * p->adj_work_cta * sizeof(float2));
+        if (!rc) rc = p->tab_rows.ensure(rows_table_bytes(p));
         if (rc == IMG2D_ENOMEM && source_mode != IMG2D_SOURCE_REUSE) {
             // too little memory for every S_l: the slab kernel
             p->adj_cache.release();
