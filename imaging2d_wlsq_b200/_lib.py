@@ -99,6 +99,8 @@ def load():
     lib.img2d_plan_kernel_ms.argtypes = [c_void_p, POINTER(ctypes.c_float)]
     lib.img2d_plan_status.restype = c_int
     lib.img2d_plan_status.argtypes = [c_void_p, c_void_p]
+    lib.img2d_plan_inject_status.restype = c_int
+    lib.img2d_plan_inject_status.argtypes = [c_void_p, c_int, c_void_p]
     lib.img2d_pack_shots.restype = c_int
     lib.img2d_pack_shots.argtypes = [c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                      c_void_p, c_void_p, POINTER(c_int), POINTER(c_double)]

@@ -649,7 +649,7 @@ struct img2d_plan {
     long long wave_elems = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool ev_recorded = false;
-    bool launched = false;  // a migration kernel has been queued (its status word is initialised)
+    bool launched = false;  // a kernel that reports to the status word, or could, has been queued
     // identity of this plan for caches keyed on it (a new plan may reuse a freed plan's address)
     const unsigned long long uid = next_uid();
     static unsigned long long next_uid()
@@ -1391,6 +1391,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         IMG2D_CUDA(cudaMemcpyAsync(p->segs.p, segs.data(), segs.size() * sizeof(int4), cudaMemcpyHostToDevice, us));
         IMG2D_CUDA(cudaMemcpyAsync(p->owner.p, owner.data(), owner.size() * sizeof(int16_t), cudaMemcpyHostToDevice, us));
         IMG2D_CUDA(cudaMemcpyAsync(p->shot_off.p, p->off.data(), p->off.size() * sizeof(long long), cudaMemcpyHostToDevice, us));
+        IMG2D_CUDA(cudaMemsetAsync(p->counter.p, 0, 2 * sizeof(int), us));
         // pageable sources: make sure the copies have read the host vectors before they go away
         IMG2D_CUDA(cudaStreamSynchronize(us));
     } else {
@@ -1399,6 +1400,8 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         IMG2D_CUDA(cudaMemcpy(p->segs.p, segs.data(), segs.size() * sizeof(int4), cudaMemcpyHostToDevice));
         IMG2D_CUDA(cudaMemcpy(p->owner.p, owner.data(), owner.size() * sizeof(int16_t), cudaMemcpyHostToDevice));
         IMG2D_CUDA(cudaMemcpy(p->shot_off.p, p->off.data(), p->off.size() * sizeof(long long), cudaMemcpyHostToDevice));
+        const int zero[2] = {0, 0};  // (a copy: complete on return, whatever stream the plan is used on)
+        IMG2D_CUDA(cudaMemcpy(p->counter.p, zero, sizeof(zero), cudaMemcpyHostToDevice));
     }
     if (p->carver && !p->rows) {
         // fixed scratch: fewer persistent CTAs when their private image partials would not fit
@@ -1470,15 +1473,18 @@ static MigrateArgs base_args(img2d_plan *p, cpx *wave, cpx *shot)
     return a;
 }
 
-// Status word of the last launch (after the work-queue counter), read on `st` after it.
+// Status word (after the work-queue counter), read on `st`.  Launches only ever set it: it keeps the
+// failure of any launch since the last reading, which clears it.
 static int read_status(img2d_plan *p, cudaStream_t st)
 {
     int status = 0;
     IMG2D_CUDA(cudaMemcpyAsync(&status, p->counter.as<int>() + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     IMG2D_CUDA(cudaStreamSynchronize(st));
-    if (status)
-        return fail(IMG2D_ECUDA, "a bounded wait in the migration kernel gave up (status " + std::to_string(status) +
-                                     "): the results of that launch are not valid");
+    if (status) {
+        IMG2D_CUDA(cudaMemsetAsync(p->counter.as<int>() + 1, 0, sizeof(int), st));
+        return fail(IMG2D_ECUDA, "a bounded wait inside a kernel of this plan gave up (status " + std::to_string(status) +
+                                     "): results since the last status check are not valid");
+    }
     return IMG2D_OK;
 }
 
@@ -1511,7 +1517,7 @@ static int launch(img2d_plan *p, MigrateArgs a, float *d_image, float *d_image_s
                   long long img_sstride, cudaStream_t st)
 {
     const size_t plane = (size_t)p->nextrap * p->nx;
-    IMG2D_CUDA(cudaMemsetAsync(p->counter.p, 0, 2 * sizeof(int), st));
+    IMG2D_CUDA(cudaMemsetAsync(p->counter.p, 0, sizeof(int), st));
     a.status = p->counter.as<int>() + 1;
     p->launched = true;
     if (d_image && p->rows) {
@@ -1902,7 +1908,7 @@ static int run_dense(int ns, int nextrap, int nz, int nx, int nf, int nt, int M,
         a.denseB = dB + first(c) * depth;
         a.image_shots = dI + (size_t)first(c) * nx;
         a.img_sstride = (long long)plane;
-        IMG2D_CUDA(cudaMemsetAsync(plan.counter.p, 0, 2 * sizeof(int), 0));
+        IMG2D_CUDA(cudaMemsetAsync(plan.counter.p, 0, sizeof(int), 0));
         return launch_kernel(&plan, a, plan.grid, 0);
     });
     const cudaError_t done = cudaDeviceSynchronize();  // nothing queued is left behind, errors or not
@@ -2223,6 +2229,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
     a.ckpt_mode = source_mode;
     a.ckpt_items = source_mode == IMG2D_SOURCE_RECOMPUTE ? nullptr : p->adj_cache.as<float2>();
     IMG2D_CUDA(cudaMemsetAsync(p->adj_counter.p, 0, sizeof(int), st));
+    p->launched = true;
     if (p->timing && !p->ev0) {
         IMG2D_CUDA(cudaEventCreate(&p->ev0));
         IMG2D_CUDA(cudaEventCreate(&p->ev1));
@@ -2243,10 +2250,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
         cfg.numAttrs = 1;
         if (p->adj_wide_fn) {
             // its bounded waits report to the plan's status word
-            int *status = p->counter.as<int>() + 1;
-            IMG2D_CUDA(cudaMemsetAsync(status, 0, sizeof(int), st));
-            p->launched = true;
-            IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_wide_fn, a, status));
+            IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_wide_fn, a, p->counter.as<int>() + 1));
         } else {
             IMG2D_CUDA(cudaLaunchKernelEx(&cfg, p->adj_fn, a));
         }
@@ -2403,6 +2407,14 @@ int img2d_plan_status(img2d_plan *p, void *stream)
     if (!p) return fail(IMG2D_EINVAL, "plan is NULL");
     if (!p->launched) return fail(IMG2D_EINVAL, "no kernel launched on this plan yet");
     return img2d::read_status(p, (cudaStream_t)stream);
+}
+
+int img2d_plan_inject_status(img2d_plan *p, int status, void *stream)
+{
+    if (!p) return fail(IMG2D_EINVAL, "plan is NULL");
+    IMG2D_CUDA(cudaMemcpyAsync(p->counter.as<int>() + 1, &status, sizeof(int), cudaMemcpyHostToDevice, (cudaStream_t)stream));
+    IMG2D_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    return IMG2D_OK;
 }
 
 int img2d_measure_fp32_peak(double *tflops)

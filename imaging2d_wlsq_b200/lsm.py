@@ -102,6 +102,13 @@ class MigrationOperator:
         self._kept = self._kept or source == "keep"
         return data
 
+    def check_status(self):
+        """Plan.check_status after the calls queued on the current stream.  migrate and demigrate (and the
+        autograd functions) do not wait for the device; the solvers and tests below, which do, check."""
+        import torch
+        if self.device.type == "cuda":
+            self.plan.check_status(torch.cuda.current_stream(self.device))
+
 
 def _functions():
     import torch
@@ -205,13 +212,16 @@ def dot_product_test(op, seed=0, data=None, refl=None, separation=0.0):
     lhs = op.image_dot(img, refl)
     rhs = op.data_dot(data, op.demigrate(refl))
     scale = np.sqrt(op.image_dot(img, img) * op.image_dot(refl, refl))
+    op.check_status()
     return lhs, rhs, abs(lhs - rhs) / max(abs(lhs), abs(rhs)), abs(lhs - rhs) / scale
 
 
 def misfit(op, refl, d_obs):
     """J(m) = 1/2 ||F* m - d_obs||^2 in float64."""
     r = op.demigrate(refl) - d_obs
-    return 0.5 * op.data_dot(r, r)
+    j = 0.5 * op.data_dot(r, r)
+    op.check_status()
+    return j
 
 
 def finite_difference_check(op, refl, d_obs, points, h):
@@ -258,6 +268,7 @@ def lsm_cg(op, d_obs, niter, refl0=None, callback=None):
         rnorm = float(np.sqrt(_allreduce_scalar(float(rr.detach()), op.group, op.device)))
         if it == niter:
             _sync(op)
+            op.check_status()
             hist.append((it, rnorm, time.perf_counter() - t0))
             m = m.detach()
             break
@@ -265,6 +276,7 @@ def lsm_cg(op, d_obs, niter, refl0=None, callback=None):
         g = m.grad.detach()
         m = m.detach()
         _sync(op)
+        op.check_status()
         hist.append((it, rnorm, time.perf_counter() - t0))
         if callback:
             callback(it, m, rnorm)
@@ -301,5 +313,6 @@ def cgls(op, d_obs, niter, refl0=None):
         p = s + (gamma_new / gamma) * p
         gamma = gamma_new
         _sync(op)
+        op.check_status()
         hist.append((it + 1, float(np.sqrt(op.data_dot(r, r))), time.perf_counter() - t0))
     return m, hist

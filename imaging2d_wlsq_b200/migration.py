@@ -202,8 +202,9 @@ class Plan:
         return v.value
 
     def check_status(self, stream=None):
-        """Raise LibraryError if a bounded wait inside the last migration kernel gave up (its results
-        are then invalid); waits for that kernel."""
+        """Raise LibraryError if a bounded wait inside a kernel of this plan gave up since the last check
+        (results since then are invalid); waits for the kernels queued on the stream.  execute() and
+        demigrate() are asynchronous and do not check by themselves."""
         check(lib().img2d_plan_status(self._h, self._stream(stream)))
 
     def shot_offset(self, s):

@@ -76,6 +76,7 @@ def _migrate_on_device(sub, device, plan_kw):
         image = torch.zeros((sub.nz, sub.nx), dtype=torch.float32, device=dev)
         plan.execute(wave, shot, image)
         torch.cuda.synchronize(dev)
+        plan.check_status()
     finally:
         plan.close()
     return image, wave, shot

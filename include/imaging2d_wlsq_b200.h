@@ -159,11 +159,13 @@ void img2d_plan_destroy(img2d_plan *plan);
  * plan, from CUDA events recorded around that launch on its stream (waits for it to finish). */
 int img2d_plan_kernel_ms(img2d_plan *plan, float *ms);
 
-/* Status of the last migration launch on this plan, read on `stream` after it (waits for it):
- * IMG2D_ECUDA if a bounded wait inside the kernel gave up (the wide migration and demigration
- * kernels; the results of that launch are then invalid), else IMG2D_OK.
- * img2d_migrate_compact checks it by itself. */
+/* Status of the migrations and demigrations launched on this plan since the last call of this
+ * function, read on `stream` after them (waits for them): IMG2D_ECUDA if a bounded wait inside one of
+ * the kernels gave up (the wide migration and demigration kernels; results since the last call are
+ * then invalid), else IMG2D_OK.  Reading clears the status.  img2d_migrate_compact checks it by itself. */
 int img2d_plan_status(img2d_plan *plan, void *stream);
+/* For tests of callers: sets the status word as a kernel whose wait gave up would. */
+int img2d_plan_inject_status(img2d_plan *plan, int status, void *stream);
 
 /* Host only (no GPU needed): the wide kernel's packing of shots into items of up to 8 lane slots.
  * windows = 0: the line packing (K <= 0: clusters just wide enough for its widest group);
