@@ -454,17 +454,28 @@ static int device_alloc(void **p, size_t n, size_t *got, int *dev)
     return IMG2D_OK;
 }
 
+// Waits for the work of all streams of the current device, as cudaFree of the block itself would: a
+// cudaFree of a small one.  cudaDeviceSynchronize would invalidate a capture that is going on in a
+// stream of the device (in another thread, or in this one in relaxed mode), where freeing is allowed.
+static bool wait_as_free_does()
+{
+    void *q = nullptr;
+    return cudaMalloc(&q, 256) == cudaSuccess && cudaFree(q) == cudaSuccess;
+}
+
 static void device_free(void *p, size_t n, int dev)
 {
     int cur = -1;
-    if (n >= kPoolMinBlock && n <= kPoolMaxBytes && cudaGetDevice(&cur) == cudaSuccess && cur == dev &&
-        cudaDeviceSynchronize() == cudaSuccess) {
+    if (n >= kPoolMinBlock && n <= kPoolMaxBytes && cudaGetDevice(&cur) == cudaSuccess && cur == dev && wait_as_free_does()) {
         DevicePool &pool = device_pool();
         std::lock_guard<std::mutex> lock(pool.mu);
-        if (pool.bytes[dev] + n <= kPoolMaxBytes) {
-            pool.blocks[dev].emplace(n, p);
-            pool.bytes[dev] += n;
-            return;
+        try {
+            if (pool.bytes[dev] + n <= kPoolMaxBytes) {
+                pool.blocks[dev].emplace(n, p);
+                pool.bytes[dev] += n;
+                return;
+            }
+        } catch (...) {  // no host memory for the entry: the block is freed
         }
     }
     cudaGetLastError();
