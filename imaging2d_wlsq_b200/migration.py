@@ -113,6 +113,13 @@ def l2_read_bandwidth_gbs():
     return v.value
 
 
+def release_cached_memory():
+    """Give back the device and page-locked memory that the library keeps between calls: the host entry's
+    plan and buffers, the blocks of closed plans and finished dense calls (up to 2 GB a device, which
+    no other allocator of the process can use meanwhile) and the upload buffers."""
+    lib().img2d_release_host_cache()
+
+
 class Plan:
     """Device-resident migration plan (torch CUDA tensors in, torch CUDA tensors out)."""
 
