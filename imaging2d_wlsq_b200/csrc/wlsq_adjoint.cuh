@@ -50,6 +50,7 @@ struct DemigrateArgs {
     float2 *work;            // per CTA: ckpt[nslab][wmax*G], slab[D][wmax*G], save[wmax*G]
     long long work_cta;      // float2 elements per CTA
     int wmax;
+    int plane;               // wide kernel: positions per CTA of a plane, the widest window's share
     int *counter;
     // source checkpoints: 0 = per CTA, recomputed in every call; 1 = computed into the per-item
     // cache ckpt_items[item][nslab][wmax*G]; 2 = read from that cache (no checkpoint pass)

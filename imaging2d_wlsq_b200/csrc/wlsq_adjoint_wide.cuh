@@ -40,6 +40,10 @@ struct DemigWideShape {
     static constexpr int RING = 8 * kRingSlots + 1;
 };
 
+// Positions of a window of W per CTA of a cluster of K: an even split in whole warps (64 positions).  In
+// units of 256, as the migration splits, a window of 300 ran 8 warps of which 5 had work.
+__host__ __device__ inline int demigw_share(int W, int K) { return (W + K * 64 - 1) / (K * 64) * 64; }
+
 // row numbers of a warp's 64 positions and MP more on either side
 __host__ __device__ inline int demigw_idx(int M) { return 64 + 2 * cluster2_mp(M); }
 
@@ -77,7 +81,7 @@ __global__ void __launch_bounds__(DemigWideShape::NW * 32, 1) demigrate_wide_ker
     const int row_bytes = a.tab_stride * 8;
     const char *tabb = reinterpret_cast<const char *>(a.tab);
     const unsigned rank0_item = map_rank(&s_item, 0);
-    const long long pe = (long long)S::PC * ROW;  // float4 per plane
+    const long long pe = (long long)a.plane * ROW;  // float4 per plane
     float4 *work = reinterpret_cast<float4 *>(a.work) + (long long)blockIdx.x * (a.work_cta / 2);
     float4 *slabbuf = work + (long long)a.nslab * pe;
     float4 *save = slabbuf + (long long)a.slab * pe;
@@ -116,8 +120,7 @@ __global__ void __launch_bounds__(DemigWideShape::NW * 32, 1) demigrate_wide_ker
         const int2 item = a.items[it];
         const GroupDesc grp = a.groups[item.x];
         const int j = item.y, u0 = grp.u0, W = grp.W;
-        // even split of the window in units of 256 positions, as in the migration
-        const int NC = min(S::PC, (W + (int)csize * 256 - 1) / ((int)csize * 256) * 256);
+        const int NC = demigw_share(W, (int)csize);
         const int c0 = (int)crank * NC;
         const int own = max(0, min(NC, W - c0));
         const bool warp_active = warp * (P * X) < NC;

@@ -1741,7 +1741,7 @@ static int demig_prepare(img2d_plan *p, int slab)
         if (nclusters <= 0) return fail(IMG2D_ECUDA, "no demigration cluster of this size fits on the device");
         grid = (int)std::min<size_t>(items.size(), (size_t)nclusters) * K;
         // float4 per plane
-        const long long pe4 = wide_fn ? (long long)DemigWideShape::PC * DemigWideShape::ROW : (long long)kDcPC * kDcQ;
+        const long long pe4 = wide_fn ? (long long)demigw_share(widest, K) * DemigWideShape::ROW : (long long)kDcPC * kDcQ;
         work_cta = 2 * (long long)(nslab + slab + 1) * pe4;
         cache_item = 2 * (long long)K * nslab * pe4;
     } else if (rows_fn) {
@@ -2236,6 +2236,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
     a.work = p->adj_work.as<float2>();
     a.work_cta = p->adj_work_cta;
     a.wmax = p->adj_wmax;
+    a.plane = p->adj_wide_fn ? demigw_share(p->adj_wmax, p->adj_cluster) : 0;
     a.counter = p->adj_counter.as<int>();
     a.ckpt_mode = source_mode;
     a.ckpt_items = source_mode == IMG2D_SOURCE_RECOMPUTE ? nullptr : p->adj_cache.as<float2>();
