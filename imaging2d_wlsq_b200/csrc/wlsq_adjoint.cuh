@@ -207,8 +207,11 @@ __device__ __forceinline__ void fir_transposed_rt(const DemigrateArgs &a, const 
 #pragma unroll
     for (int jj = 0; jj < X; ++jj) {
         float r0 = 0.f, i0 = 0.f;
-        for (int k = L - 1; k >= 0; --k) {  // inputs in increasing position, as in fir_transposed
-            const int xi = xb + jj + M - k;
+        // inputs in increasing position, as in fir_transposed.  Counted up and in fours: the loop over taps
+        // counted down was not unrolled (4 shots of 2351 positions, 47 taps: 123 ms against 98).
+#pragma unroll 4
+        for (int i = 0; i < L; ++i) {
+            const int xi = xb + jj - M + i, k = L - 1 - i;
             const float2 v = src[pad_slot(xi, X) * G + q];
             int xm = u0 + xi - Mp;
             xm = xm < 0 ? 0 : (xm < a.nx ? xm : a.nx - 1);

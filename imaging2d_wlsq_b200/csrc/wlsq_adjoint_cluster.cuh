@@ -64,8 +64,9 @@ __device__ __forceinline__ void fir2_transposed(const DemigrateArgs &a, const fl
 #pragma unroll
     for (int jj = 0; jj < X; ++jj) {
         acc[jj][0] = acc[jj][1] = acc[jj][2] = acc[jj][3] = 0.f;
-        for (int k = 2 * M; k >= 0; --k) {
-            const int d = jj + M - k;  // input offset from the block start
+#pragma unroll 4
+        for (int i = 0; i <= 2 * M; ++i) {
+            const int d = jj - M + i, k = 2 * M - i;  // input offset from the block start, its tap
             const int xm = min(max(xm0 + d, 0), a.nx - 1);
             const cpx f = a.tab[(long long)sidx[xm] * a.tab_stride + k];
             mac2(acc[jj], f.re, f.im, src[(pb + d) * kDcQ]);
