@@ -682,6 +682,7 @@ struct img2d_plan {
     int block = 256;                  // threads per CTA of the chosen kernel
     bool allow_rows = true, rows_tab_set = false;
     bool rows = false;                // the row-split kernel (its table order, visit counts per CTA)
+    img2d::RowsStarts row_starts{{0, 0, 0, 0}, 0};  // set by plan_row_starts on its first call
     int variant = -1;                 // index into the cluster2 variant table
     int tab16 = 0;                    // operator table storage: 0 FP32, 1 FP16, 2 BF16
     const char *kname = "";           // name of the chosen kernel
@@ -1451,6 +1452,13 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
     return IMG2D_OK;
 }
 
+// The search takes 10 to 550 us on the host: once per plan, not at every launch.
+static const RowsStarts &plan_row_starts(img2d_plan *p)
+{
+    if (!p->row_starts.apart) p->row_starts = rows_starts(p->L);
+    return p->row_starts;
+}
+
 static MigrateArgs base_args(img2d_plan *p, cpx *wave, cpx *shot)
 {
     MigrateArgs a{};
@@ -1470,7 +1478,7 @@ static MigrateArgs base_args(img2d_plan *p, cpx *wave, cpx *shot)
     a.tab16 = p->tab16buf.p;
     if (p->rows) {
         a.tab_rows = p->tab_rows.p;
-        const RowsStarts rs = rows_starts(p->L);
+        const RowsStarts &rs = plan_row_starts(p);
         for (int i = 0; i < 4; ++i) a.row_start[i] = rs.s[i];
         a.row_apart = rs.apart;
     }
@@ -1582,7 +1590,7 @@ static int set_rows_table(img2d_plan *p, cudaStream_t st)
     const int rc = p->tab_rows.ensure(rows_table_bytes(p));
     if (rc) return rc;
     rows_table_kernel<<<(int)std::min<long long>((floats / 2 + 255) / 256, 148 * 8), 256, 0, st>>>(
-        p->tabF.as<cpx>(), two ? p->tabB.as<cpx>() : nullptr, p->tab_stride, p->L, rows_np(p->L), rows_starts(p->L),
+        p->tabF.as<cpx>(), two ? p->tabB.as<cpx>() : nullptr, p->tab_stride, p->L, rows_np(p->L), plan_row_starts(p),
         p->nk, p->tab_rows.as<float>());
     IMG2D_CUDA(cudaGetLastError());
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -2272,7 +2280,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
         ra.d = a;
         if (!p->adj_full_cache) ra.d.ckpt_mode = IMG2D_SOURCE_RECOMPUTE;
         ra.tab_rows = p->tab_rows.p;
-        const RowsStarts rs = rows_starts(p->L);
+        const RowsStarts &rs = plan_row_starts(p);
         for (int i = 0; i < 4; ++i) ra.row_start[i] = rs.s[i];
         ra.row_apart = rs.apart;
         ra.planes = ra.d.ckpt_mode ? p->adj_cache.p : p->adj_work.p;
