@@ -135,6 +135,24 @@ static RowsLaunch rows_launch(int G, int W, int L, bool two, long long n_items, 
     return best;
 }
 
+// Time at which the last of nf items of each cost is done, taken in order of falling cost by `workers`.
+static double queue_time(std::vector<double> cost, int nf, int workers)
+{
+    std::sort(cost.begin(), cost.end(), std::greater<double>());
+    const double sum = std::accumulate(cost.begin(), cost.end(), 0.0) * nf;
+    const long long n = (long long)cost.size() * nf;
+    if (n <= workers) return cost[0];
+    if (n > 64ll * workers) return sum / workers + 0.5 * cost.back();
+    std::vector<double> heap(workers, 0.0);  // when each worker is free, the earliest first
+    for (double c : cost)
+        for (int j = 0; j < nf; ++j) {
+            std::pop_heap(heap.begin(), heap.end(), std::greater<double>());
+            heap.back() += c;
+            std::push_heap(heap.begin(), heap.end(), std::greater<double>());
+        }
+    return *std::max_element(heap.begin(), heap.end());
+}
+
 static KernelFn find_generic(int G, int mode)
 {
 #define IMG2D_GEN(GG)                                                        \
@@ -682,7 +700,7 @@ struct img2d_plan {
     int block = 256;                  // threads per CTA of the chosen kernel
     bool allow_rows = true, rows_tab_set = false;
     bool rows = false;                // the row-split kernel (its table order, visit counts per CTA)
-    img2d::RowsStarts row_starts{{0, 0, 0, 0}, 0};  // set by plan_row_starts on its first call
+    img2d::RowsStarts row_starts{{0, 0, 0, 0}, 0, 0.0};  // set by plan_row_starts on its first call
     int variant = -1;                 // index into the cluster2 variant table
     int tab16 = 0;                    // operator table storage: 0 FP32, 1 FP16, 2 BF16
     const char *kname = "";           // name of the chosen kernel
@@ -1035,6 +1053,13 @@ static double pack_windows_best(const img2d_plan *p, int G, int K, std::vector<G
     return best;
 }
 
+// The search takes 10 to 550 us on the host: once per plan, not at every launch.
+static const RowsStarts &plan_row_starts(img2d_plan *p)
+{
+    if (!p->row_starts.apart) p->row_starts = rows_starts(p->L);
+    return p->row_starts;
+}
+
 static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf, int nt, int M,
                       int nk, const int *shot_x0, const int *shot_nx, int flags, int mode)
 {
@@ -1205,10 +1230,12 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                              : 0;
         want_wide = p->n_slots < 12 || busy < nsm * 96 / 100;
     }
-    // The row-split kernel instead: always for a table pair, and for single tables where it is
+    // The row-split kernel instead: always for a table pair and for fewer than 6 slots, else where it is
     // estimated faster than the kernel chosen below.  Surveys of 12 slots or more are only considered
-    // when its items fill the SMs (the estimates are made for that).
+    // when its items fill the SMs, with fewer than 16 frequencies (the least the estimates below are
+    // fitted to) four times over.
     int rows_G = 1;
+    std::vector<int> rows_W;  // its items' windows
     RowsLaunch rows_l{1, 1e30};
     if (p->allow_rows && mode != OP_DENSE && !explicit_kernel && find_rows(1, p->L, mode == OP_TWO)) {
         int smem_sm = 0;
@@ -1217,33 +1244,16 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             const int widest = make_groups(G);
             if (rows_smem_bytes(G, widest, p->L) + static_reserve > (size_t)smem_optin) continue;
             const long long n = (long long)groups.size() * nf;
-            if (p->n_slots >= 12 && mode == OP_CONJ && n < nsm) continue;
+            if (p->n_slots >= 12 && mode == OP_CONJ && n < nsm * (nf < 16 ? 4 : 1)) continue;
             const RowsLaunch r = rows_launch(G, widest, p->L, mode == OP_TWO, n, nsm, smem_sm);
             if (r.us < rows_l.us) {
                 rows_l = r;
                 rows_G = G;
+                rows_W.clear();
+                for (const GroupDesc &g : groups) rows_W.push_back(g.W);
             }
         }
-        if (rows_l.us < 1e30) {
-            if (mode == OP_TWO || p->n_slots < 6) {
-                p->rows = true;
-            } else {
-                // Time of a depth step of the wide kernel (8 slots x up to 1024 positions per CTA) or of the
-                // 16-slot one (up to 512), in microseconds, for a CTA with all warps busy: fitted on a
-                // B200 to 25 to 55 taps, windows of 256 to 1024 positions.  Clusters of three and more
-                // leave about 9% of the SMs idle.  The row-split estimate is 8% low on average (16
-                // surveys of 7 to 179 shots).
-                const bool wide = want_wide;
-                const int G = wide ? WideShape::G : 16, pc = wide ? WideShape::PC : 512;
-                const int widest = make_groups(G), K = (widest + pc - 1) / pc;
-                const int nc = std::min(pc, (widest + K * 256 - 1) / (K * 256) * 256);
-                const double item = wide ? 0.344 * (p->L + 15) * wide_item_cost(nc, 1)
-                                         : 0.375 * (p->L + 7.4) * (nc == pc ? 1.0 : 0.57);
-                const int clusters = std::max(1, (K > 2 ? nsm * 91 / 100 : nsm) / K);
-                const double waves = (double)groups.size() * nf / clusters;
-                p->rows = 1.08 * rows_l.us < item * (waves <= 4.0 ? std::ceil(waves) : waves + 0.5);
-            }
-        }
+        p->rows = rows_l.us < 1e30 && (mode == OP_TWO || p->n_slots < 6);
     }
     // The 16-slot default: the wide kernel's step with 8 lanes per group (16 slots x 512 positions per
     // CTA, clusters as cluster2's), reported as the cluster2 variant after those of the table.
@@ -1296,8 +1306,48 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             p->kname = "migrate_cluster";
         }
     }
+    if (!p->rows && rows_l.us < 1e30 && !p->cluster) p->rows = true;  // a lane per output: two to six times slower
+    if (!p->rows && rows_l.us < 1e30) {
+        // Either kernel's items, widest first, through the queue of its CTAs or clusters.  Microseconds per
+        // depth step and item, fitted on a B200 to 316 surveys of 6 to 256 shots, 16 to 256 frequencies,
+        // 100 to 4096 positions, 19 to 55 taps: the wide kernel (8 slots) and the 16-slot one within 4%
+        // (standard deviation), the row-split one within 5 (a slot) and 6.5% (two).  Two of the
+        // surveys come out slower than without the row-split kernel, by 4 and 5%; taken in waves of
+        // the widest window it was twelve, by up to 19%.
+        const KernelFn rfn = find_rows(rows_G, p->L, mode == OP_TWO);
+        const size_t rsmem = rows_smem_bytes(rows_G, *std::max_element(rows_W.begin(), rows_W.end()), p->L);
+        int per_sm = 0;
+        IMG2D_CUDA(cudaFuncSetAttribute(rfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
+        IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rfn, 32 * rows_l.warps, rsmem));
+        const int slots = (int)std::min<long long>((long long)rows_W.size() * nf, (long long)nsm * std::max(per_sm, 1));
+        const int per = (slots + nsm - 1) / nsm;  // CTAs that share an SM
+        const int q = rows_np(p->L);
+        // 3 pairs of taps cost as much as 4: their second chunk of 2 taps is a load of its own
+        const double round = rows_G == 1 ? 0.11 + 0.0615 * q
+                                         : (0.123 + 0.103 * (q == 3 ? 4 : q)) * std::pow(plan_row_starts(p).passes, 0.117) *
+                                               (per > 1 ? 0.905 : 1.0);
+        std::vector<double> mine, other;
+        for (int W : rows_W) {
+            const int nwb = (W + kRowsWarpPos - 1) / kRowsWarpPos;
+            const int rounds = (nwb + rows_l.warps - 1) / rows_l.warps;
+            const double active = (double)per * nwb / rounds;  // warps on the SM
+            mine.push_back(round * (rounds * (1.0 + 0.25 * active) + (rows_G == 1 ? 1.0 : 0.6)));
+        }
+        const bool wide = p->G == WideShape::G;
+        const int pc = wide ? WideShape::PC : 512, K = p->cluster;
+        for (const GroupDesc &g : groups) {
+            const double share = (double)std::min(pc, (g.W + K * 256 - 1) / (K * 256) * 256) / pc;
+            other.push_back(wide ? 1.4 + 0.083 * p->L + (4.7 + 0.25 * p->L) * share
+                                 : 1.5 + 0.02 * p->L + (0.85 + 0.35 * p->L) * share);
+        }
+        const int clusters = std::max(1, clusters_that_fit((const void *)p->fn, K, p->block, p->smem));
+        p->rows = queue_time(mine, nf, slots) < queue_time(other, nf, clusters);
+    }
     if (p->rows) {
         p->cluster = 0;
+        p->variant = -1;
+        p->packing = "lines";
+        p->pack_cost = 0.0;
         p->G = rows_G;
         p->fixed = true;
         p->fn = find_rows(rows_G, p->L, mode == OP_TWO);
@@ -1450,13 +1500,6 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         if ((rc = p->tab_rows.ensure(rows_tab_b))) return rc;
     }
     return IMG2D_OK;
-}
-
-// The search takes 10 to 550 us on the host: once per plan, not at every launch.
-static const RowsStarts &plan_row_starts(img2d_plan *p)
-{
-    if (!p->row_starts.apart) p->row_starts = rows_starts(p->L);
-    return p->row_starts;
 }
 
 static MigrateArgs base_args(img2d_plan *p, cpx *wave, cpx *shot)

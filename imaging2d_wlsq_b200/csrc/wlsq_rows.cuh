@@ -54,12 +54,13 @@ __host__ __device__ constexpr int rows_pad(int x) { return x + (x >> 3); }
 // 3.42 against 3.68 ms for one shot of 1024 x 500, 256 frequencies).
 struct RowsStarts {
     int s[4];
-    int apart;  // 1, 2 or 4
+    int apart;      // 1, 2 or 4
+    double passes;  // of a quarter warp's read
 };
 inline RowsStarts rows_starts(int L)
 {
     const int X = kRowsX, Q = 2 * rows_np(L);
-    RowsStarts best{{0, 0, 0, 0}, 1};
+    RowsStarts best{{0, 0, 0, 0}, 1, 1.0};
     int best_cost = 1 << 30;
     for (int apart = 1; apart <= 4; apart *= 2)
         for (int s3 = L - Q; s3 <= L - Q + 1 && s3 <= 3 * Q; ++s3)
@@ -67,7 +68,8 @@ inline RowsStarts rows_starts(int L)
                 for (int s2 = s1; s2 <= s1 + Q && s2 <= s3; ++s2) {
                     if (s3 - s2 > Q) continue;
                     const int s[4] = {0, s1, s2, s3};
-                    int cost = (s3 > L - Q ? 3 : 0) + (apart > 1 ? 1 : 0);
+                    const int extra = (s3 > L - Q ? 3 : 0) + (apart > 1 ? 1 : 0);
+                    int cost = extra;
                     for (int x = 0; x < 64; ++x) {
                         int at[8], banks[8] = {}, worst = 0;
                         for (int i = 0; i < 8; ++i) {
@@ -80,7 +82,7 @@ inline RowsStarts rows_starts(int L)
                     }
                     if (cost < best_cost) {
                         best_cost = cost;
-                        best = RowsStarts{{s[0], s[1], s[2], s[3]}, apart};
+                        best = RowsStarts{{s[0], s[1], s[2], s[3]}, apart, (cost - extra) / 64.0};
                     }
                 }
     return best;
