@@ -2774,8 +2774,9 @@ int img2d_source_spectra(int ns, int nt, int nx, int nf, int nt_rows, double dt,
         return img2d_records_to_spectra(ns, nt, nx, nf, nt_rows, d_t, shot_x0, shot_nx, d_out, stream);
     }
     const int nsup = std::min(nt, (int)span), kp = (nf + kSrcK - 1) / kSrcK * kSrcK;
-    int dev = 0;
+    int dev = 0, nsm = 0;
     IMG2D_CUDA(cudaGetDevice(&dev));
+    IMG2D_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     std::lock_guard<std::mutex> lock(g_front_mu);
     FrontScratch &fs = g_front[dev];
     const size_t nw = ((size_t)nt + 1) / 2 * 2, nu = (size_t)nsup * kp;
@@ -2789,7 +2790,11 @@ int img2d_source_spectra(int ns, int nt, int nx, int nf, int nt_rows, double dt,
         const int n = std::min(kSpecShots, ns - s0);
         SpecShots sh = spec_shots(s0, n, x0, w, off);
         for (int i = 0; i < n; ++i) sh.sx[i] = src_x[s0 + i];
-        source_spectra_kernel<<<dim3((nx + kSrcCols - 1) / kSrcCols, n, nf > 64 ? 2 : 1), 256, smem, st>>>(sh, nt, nx, nf, nsup, kp, dt, x_first, dx,
+        // the 64 rows that a CTA takes at a time are shared out over two CTAs, over more where the
+        // SMs would be left without (each forms the wavelets anew)
+        const int cols = (nx + kSrcCols - 1) / kSrcCols;
+        const int parts = std::min((nf + 63) / 64, std::max(2, 2 * nsm / (cols * n)));
+        source_spectra_kernel<<<dim3(cols, n, parts), 256, smem, st>>>(sh, nt, nx, nf, nsup, kp, dt, x_first, dx,
                                                                          depth_offset, v, fpeak, tw, W, U, (cpx *)d_out);
         IMG2D_CUDA(cudaGetLastError());
     }
