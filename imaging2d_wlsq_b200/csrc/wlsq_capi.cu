@@ -219,6 +219,12 @@ struct DemigKernel {
 #define IMG2D_DEMIG_G(G) IMG2D_DEMIG(G, 0), IMG2D_DEMIG(G, 25), IMG2D_DEMIG(G, 31), IMG2D_DEMIG(G, 35), IMG2D_DEMIG(G, 55)
 static const DemigKernel kDemig[] = {IMG2D_DEMIG_G(2), IMG2D_DEMIG_G(4), IMG2D_DEMIG_G(8)};
 
+// Cluster demigration with unrolled steps.
+static DemigFn find_demig_cluster(int L)
+{
+    return L == 25 ? demigrate_cluster_kernel<25> : (L == 31 ? demigrate_cluster_kernel<31> : (L == 35 ? demigrate_cluster_kernel<35> : nullptr));
+}
+
 // Row-split demigration kernels by slots per item and tap pairs per lane.
 struct DemigRowsKernel {
     int NS, np;
@@ -1701,44 +1707,73 @@ static int demig_prepare(img2d_plan *p, int slab)
     bool ring = false;
     DemigFn fn = nullptr;
     size_t smem = 0;
-    // With enough slots to fill items of 16: the wide kernel (1024 positions per CTA; 7 to 65 taps), or the
-    // cluster kernel (512 positions, any length), where the widest window fits 16 CTAs; otherwise the
-    // row-split kernel or the single-CTA one.
+    // With enough slots to fill items of 16: the wide kernel (up to 1024 positions per CTA; 7 to 65 taps) or
+    // the cluster kernel (512 positions, any length), where the widest window fits 16 CTAs; otherwise
+    // the row-split kernel or the single-CTA one.
+    //
+    // The wide kernel's windows may be spread over more CTAs than they need, and the cluster kernel has
+    // unrolled instances for 25, 31 and 35 taps.  Both are chosen by the time of their items through the
+    // queue, in microseconds per depth step of a call that recomputes its source (within 6% of 110
+    // calls on a B200, 12 to 189 shots of 100 to 3300 positions; the cluster kernel at run-time
+    // lengths takes 1.5 to 5 times as long; in clusters less than 512 positions a CTA are no faster).  A lane of the wide kernel has four slots and a warp twice
+    // the positions, so windows of 400 to 512 leave it half its warps: 13 shots of 437, 170 frequencies,
+    // 35 taps 3.03 ms, the cluster kernel 2.91.
     void (*wide_fn)(DemigrateArgs, int *) = nullptr;
-    if (p->adj_allow_wide && p->n_slots >= 12 && !(p->flags & IMG2D_FLAG_NO_CLUSTER) && p->L >= 7 &&
-        demigw_smem_bytes(p->M) + static_reserve <= (size_t)smem_optin) {
+    const bool slots16 = p->n_slots >= 12 && !(p->flags & IMG2D_FLAG_NO_CLUSTER);
+    const DemigFn ring_fn = slots16 && !(p->flags & IMG2D_FLAG_DEMIG_NO_RING) ? find_demig_cluster(p->L) : nullptr;
+    auto cluster_fits = [&](DemigFn f, int k, size_t bytes) {
+        return f && bytes + static_reserve <= (size_t)smem_optin &&
+               (k <= 8 || (k <= kMaxCluster && clusters_that_fit((const void *)f, k, kDcNW * 32, bytes) > 0));
+    };
+    if (p->adj_allow_wide && slots16 && p->L >= 7 && demigw_smem_bytes(p->M) + static_reserve <= (size_t)smem_optin) {
         widest = pack_groups(p, DemigWideShape::G, groups, segs, owner);
-        int k = (widest + DemigWideShape::PC - 1) / DemigWideShape::PC;
         // operators of less than 17 taps need few pairs per step: the wait for the ring's first copies
         // would be most of it
         const bool wring = !(p->flags & IMG2D_FLAG_DEMIG_NO_RING) && p->L >= 17;
         auto wf = wring ? demigrate_wide_kernel<true> : demigrate_wide_kernel<false>;
         const size_t wsmem = demigw_smem_bytes(p->M);
-        // few items: windows are spread over more CTAs than they need, down to 256 positions each
-        auto fits = [&](int c) {
-            return c <= 8 || (c <= kMaxCluster && clusters_that_fit((const void *)wf, c, DemigWideShape::NW * 32, wsmem) > 0);
-        };
-        while ((long long)groups.size() * p->nf * k * 2 <= nsm && widest / (2 * k) >= 256 && fits(2 * k)) k *= 2;
-        if (fits(k)) {
-            K = k;
+        const int least = (widest + DemigWideShape::PC - 1) / DemigWideShape::PC;
+        double best = 1e30;
+        for (int k = least; k == least || (k <= 8 && widest / k >= 256); ++k) {
+            // (no more planes than 512 positions per CTA would have)
+            if (k > least && k * demigw_share(widest, k) > (widest + 511) / 512 * 512) continue;
+            const int n = k <= kMaxCluster ? clusters_that_fit((const void *)wf, k, DemigWideShape::NW * 32, wsmem) : 0;
+            if (n <= 0) continue;
+            std::vector<double> cost;
+            for (const GroupDesc &g : groups)
+                cost.push_back(10.2 + (k > 1 ? 0.52 : 0.43) * p->L +
+                               (0.0045 + 0.00066 * p->L) * std::max(k > 1 ? 512 : 0, demigw_share(g.W, k)));
+            const double t = queue_time(cost, p->nf, n);
+            if (t < best) {
+                best = t;
+                K = k;
+            }
+        }
+        const int kc = (widest + kDcPC - 1) / kDcPC;
+        const size_t csmem = demigc_ring_smem_bytes(p->M);
+        if (K && cluster_fits(ring_fn, kc, csmem)) {
+            const std::vector<double> cost(groups.size(), (kc > 1 ? 10.0 : 9.0) + 0.81 * p->L);
+            const int n = clusters_that_fit((const void *)ring_fn, kc, kDcNW * 32, csmem);
+            if (n > 0 && queue_time(cost, p->nf, n) < best) K = 0;
+        }
+        if (K) {
             G = DemigWideShape::G;
             wide_fn = wf;
             smem = wsmem;
             ring = wring;
         }
     }
-    if (!K && p->n_slots >= 12 && !(p->flags & IMG2D_FLAG_NO_CLUSTER)) {
+    if (!K && slots16) {
         widest = pack_groups(p, 16, groups, segs, owner);
         const int k = (widest + kDcPC - 1) / kDcPC;
-        const DemigFn cfn = demigrate_cluster_kernel;
-        const size_t csmem = demigc_smem_bytes(p->M);
-        if (csmem + static_reserve <= (size_t)smem_optin) {
-            if (k <= 8 || (k <= kMaxCluster && clusters_that_fit((const void *)cfn, k, kDcNW * 32, csmem) > 0)) {
-                K = k;
-                G = 16;
-                fn = cfn;
-                smem = csmem;
-            }
+        for (DemigFn f : {ring_fn, (DemigFn)demigrate_cluster_kernel<0>}) {
+            const size_t bytes = f == ring_fn ? demigc_ring_smem_bytes(p->M) : demigc_smem_bytes(p->M);
+            if (K || !cluster_fits(f, k, bytes)) continue;
+            K = k;
+            G = 16;
+            fn = f;
+            smem = bytes;
+            ring = f == ring_fn;
         }
     }
     // Fewer slots: the row-split kernel, which keeps every S_l, where its shared memory fits.
@@ -2348,10 +2383,10 @@ int img2d_plan_describe_demigration(const img2d_plan *p, char *buf, int buflen)
     snprintf(buf, buflen,
              "{\"kernel\": \"%s\", \"cluster\": %d, \"G\": %d, \"X\": 8, \"L\": %d, \"grid\": %d, \"block\": %d, "
              "\"smem\": %zu, \"items\": %d, \"max_union_width\": %d, \"slab\": %d, \"slabs\": %d, "
-             "\"workspace_bytes\": %zu, \"source_cache_bytes\": %zu, \"ring\": %s}",
+             "\"workspace_bytes\": %zu, \"source_cache_bytes\": %zu, \"ring\": %s, \"wide\": %s}",
              p->adj_rows ? "demigrate_rows" : (p->adj_cluster ? "demigrate_cluster" : "demigrate"), p->adj_cluster, p->adj_G, p->L, p->adj_grid,
              p->adj_block, p->adj_smem, p->adj_items_n, p->adj_wmax, p->adj_slab,
-             p->adj_nslab, p->adj_work.bytes, p->adj_cache.bytes, p->adj_ring ? "true" : "false");
+             p->adj_nslab, p->adj_work.bytes, p->adj_cache.bytes, p->adj_ring ? "true" : "false", p->adj_wide_fn ? "true" : "false");
     return IMG2D_OK;
 }
 
