@@ -2276,12 +2276,19 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
     if (source_mode == IMG2D_SOURCE_REUSE && !p->adj_cache_valid)
         return fail(IMG2D_EINVAL, "no kept source checkpoints on this plan (call with IMG2D_SOURCE_KEEP first, "
                                   "after the last set_model, with the same slab depth)");
+    int rows_grid = p->adj_grid;
     if (p->adj_rows) {
         rc = IMG2D_OK;
         if (source_mode == IMG2D_SOURCE_KEEP)
             rc = p->adj_cache.ensure(p->adj_full_cache ? (size_t)p->adj_items_n * p->adj_cache_item * sizeof(float2) : 16);
-        if (!rc && !(p->adj_full_cache && source_mode != IMG2D_SOURCE_RECOMPUTE))
-            rc = p->adj_work.ensure((size_t)p->adj_grid * p->adj_work_cta * sizeof(float2));
+        if (!rc && !(p->adj_full_cache && source_mode != IMG2D_SOURCE_RECOMPUTE)) {
+            rc = p->adj_work.ensure((size_t)rows_grid * p->adj_work_cta * sizeof(float2));
+            // beside a kept source, which the slab kernel could not use: fewer CTAs
+            while (rc == IMG2D_ENOMEM && p->adj_cache_valid && p->adj_full_cache && rows_grid > 1) {
+                rows_grid /= 2;
+                rc = p->adj_work.ensure((size_t)rows_grid * p->adj_work_cta * sizeof(float2));
+            }
+        }
         if (!rc) rc = p->tab_rows.ensure(rows_table_bytes(p));
         if (rc == IMG2D_ENOMEM && source_mode != IMG2D_SOURCE_REUSE) {
             // too little memory for every S_l: the slab kernel
@@ -2363,7 +2370,7 @@ int img2d_plan_demigrate(img2d_plan *p, const float *d_refl, const img2d_c64 *d_
         ra.row_apart = rs.apart;
         ra.planes = ra.d.ckpt_mode ? p->adj_cache.p : p->adj_work.p;
         ra.plane = rows_adj_wp(p->adj_wmax);
-        p->adj_rows_fn<<<p->adj_grid, p->adj_block, p->adj_smem, st>>>(ra);
+        p->adj_rows_fn<<<rows_grid, p->adj_block, p->adj_smem, st>>>(ra);
     } else {
         p->adj_fn<<<p->adj_grid, p->adj_block, p->adj_smem, st>>>(a);
     }
