@@ -112,18 +112,18 @@ static KernelFn find_rows(int G, int L, bool two)
 // n_items items of windows up to W.  A step of a CTA is `rounds` blocks per warp, each taking
 // 0.45 us (1 + k / 6) with k warps on the SM, times 1.45 for two slots (fitted on a B200, 31 taps,
 // one table: 3 to 16 warps per SM; within 15% on the cases it was checked on); items beyond what is
-// resident run in further waves.
+// resident run in further waves.  At most `most` CTAs share an SM.
 struct RowsLaunch {
     int warps;
     double us;
 };
-static RowsLaunch rows_launch(int G, int W, int L, bool two, long long n_items, int nsm, size_t smem_sm)
+static RowsLaunch rows_launch(int G, int W, int L, bool two, long long n_items, int nsm, size_t smem_sm, int most)
 {
     const int nwb = (W + kRowsWarpPos - 1) / kRowsWarpPos;
     const size_t smem = rows_smem_bytes(G, W, L) + 1024;
     RowsLaunch best{1, 1e30};
     for (int w = 1; w <= std::min(nwb, kRowsThreads / 32); ++w) {
-        const long long c = std::min<long long>(16 / w, (long long)(smem_sm / smem));  // 128 registers a thread
+        const long long c = std::min<long long>({16 / w, (long long)(smem_sm / smem), most});  // 128 registers a thread
         if (c < 1) continue;
         const int rounds = (nwb + w - 1) / w;
         auto wave = [&](long long per_sm) { return rounds * 0.45 * (1.0 + per_sm * w / 6.0); };
@@ -1242,6 +1242,9 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
     // fitted to) four times over.
     int rows_G = 1;
     std::vector<int> rows_W;  // its items' windows
+    // Its CTAs have a partial image and compensation each.  Those of several CTAs per SM take at most 8 GB:
+    // 5 shots of 600 traces over 4096 x 1000, 256 frequencies, took 14.5 GB.
+    const int rows_most = (int)std::max<size_t>(1, (8ull << 30) / ((size_t)nsm * nextrap * nx * 8));
     RowsLaunch rows_l{1, 1e30};
     if (p->allow_rows && mode != OP_DENSE && !explicit_kernel && find_rows(1, p->L, mode == OP_TWO)) {
         int smem_sm = 0;
@@ -1251,7 +1254,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
             if (rows_smem_bytes(G, widest, p->L) + static_reserve > (size_t)smem_optin) continue;
             const long long n = (long long)groups.size() * nf;
             if (p->n_slots >= 12 && mode == OP_CONJ && n < nsm * (nf < 16 ? 4 : 1)) continue;
-            const RowsLaunch r = rows_launch(G, widest, p->L, mode == OP_TWO, n, nsm, smem_sm);
+            const RowsLaunch r = rows_launch(G, widest, p->L, mode == OP_TWO, n, nsm, smem_sm, rows_most);
             if (r.us < rows_l.us) {
                 rows_l = r;
                 rows_G = G;
@@ -1325,7 +1328,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         int per_sm = 0;
         IMG2D_CUDA(cudaFuncSetAttribute(rfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
         IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rfn, 32 * rows_l.warps, rsmem));
-        const int slots = (int)std::min<long long>((long long)rows_W.size() * nf, (long long)nsm * std::max(per_sm, 1));
+        const int slots = (int)std::min<long long>((long long)rows_W.size() * nf, (long long)nsm * std::max(std::min(per_sm, rows_most), 1));
         const int per = (slots + nsm - 1) / nsm;  // CTAs that share an SM
         const int q = rows_np(p->L);
         // 3 pairs of taps cost as much as 4: their second chunk of 2 taps is a load of its own
@@ -1424,7 +1427,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         int per_sm = 0;
         IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p->fn, p->block, p->smem));
         if (per_sm <= 0) return fail(IMG2D_ECUDA, "the row-split kernel does not fit on an SM");
-        p->grid = std::min(p->n_items, nsm * per_sm);
+        p->grid = std::min(p->n_items, nsm * std::min(per_sm, rows_most));
     } else {
         p->grid = std::min(p->n_items, nsm);
     }
