@@ -543,9 +543,15 @@ static int upload(const std::vector<UploadPiece> &pieces, int groups, cudaStream
 {
     size_t total = 0;
     for (const UploadPiece &u : pieces) total += u.n;
-    cudaPointerAttributes at{};
-    bool staged = total >= 4 * kStagePiece &&
-                  (cudaPointerGetAttributes(&at, pieces[0].src) != cudaSuccess || at.type == cudaMemoryTypeUnregistered);
+    // staged from pageable memory only, every array of the first group: the workers copy on the host
+    bool staged = total >= 4 * kStagePiece;
+    const unsigned char *next_src = nullptr;
+    for (size_t i = 0; staged && i < pieces.size() && pieces[i].group == pieces[0].group; ++i) {
+        cudaPointerAttributes at{};
+        if (pieces[i].src != next_src && cudaPointerGetAttributes(&at, pieces[i].src) == cudaSuccess)
+            staged = at.type == cudaMemoryTypeUnregistered;
+        next_src = (const unsigned char *)pieces[i].src + pieces[i].n;
+    }
     cudaGetLastError();
     StageRing &ring = stage_ring();
     std::unique_lock<std::mutex> lock(ring.mu, std::defer_lock);
