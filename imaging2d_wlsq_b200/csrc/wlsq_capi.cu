@@ -710,7 +710,7 @@ struct img2d_plan {
     std::vector<int> group_order;  // migration groups, widest first (the order of the item queue)
     int cluster = 0;  // CTAs per cluster of the cluster kernel, 0 = single-CTA kernels
     int block = 256;                  // threads per CTA of the chosen kernel
-    bool allow_rows = true, rows_tab_set = false;
+    bool rows_tab_set = false;        // tab_rows holds the tables of the last set_model
     bool rows = false;                // the row-split kernel (its table order, visit counts per CTA)
     img2d::RowsStarts row_starts{{0, 0, 0, 0}, 0, 0.0};  // set by plan_row_starts on its first call
     int variant = -1;                 // index into the cluster2 variant table
@@ -1252,7 +1252,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
     // 5 shots of 600 traces over 4096 x 1000, 256 frequencies, took 14.5 GB.
     const int rows_most = (int)std::max<size_t>(1, (8ull << 30) / ((size_t)nsm * nextrap * nx * 8));
     RowsLaunch rows_l{1, 1e30};
-    if (p->allow_rows && mode != OP_DENSE && !explicit_kernel && find_rows(1, p->L, mode == OP_TWO)) {
+    if (mode != OP_DENSE && !explicit_kernel && find_rows(1, p->L, mode == OP_TWO)) {
         int smem_sm = 0;
         IMG2D_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
         for (int G = 1; G <= std::min(2, p->n_slots); ++G) {
@@ -1441,19 +1441,6 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
     int rc;
     const size_t plane = (size_t)nextrap * nx;
     const size_t rows_tab_b = p->rows ? (size_t)nk * rows_row_floats(p->L, mode == OP_TWO) * sizeof(float) : 0;
-    if (p->carver && p->rows) {
-        // fixed scratch: the row-split kernel only where the partial images of all its CTAs fit
-        const size_t need = items.size() * sizeof(int2) + groups.size() * sizeof(GroupDesc) +
-                            segs.size() * sizeof(int4) + owner.size() * sizeof(int16_t) +
-                            p->off.size() * sizeof(long long) + (size_t)p->grid * sizeof(int) +
-                            (size_t)nf * nextrap * ((nx + 7) / 8 * 8) * sizeof(uint16_t) + rows_tab_b +
-                            (size_t)nk * ((p->L + 1) / 2 * 2) * sizeof(cpx) * (mode == OP_TWO ? 2 : 1) +
-                            (size_t)p->grid * plane * sizeof(float) * (p->n_items > p->grid ? 2 : 1) + 16 * 256;
-        if (need > p->carver->cap - p->carver->used) {
-            p->allow_rows = p->rows = false;
-            return build_plan(p, ns, nextrap, nz, nx, nf, nt, M, nk, shot_x0, shot_nx, flags, mode);
-        }
-    }
     if ((rc = p->items.ensure(items.size() * sizeof(int2)))) return rc;
     if ((rc = p->groups.ensure(groups.size() * sizeof(GroupDesc)))) return rc;
     if ((rc = p->segs.ensure(segs.size() * sizeof(int4)))) return rc;
@@ -1480,7 +1467,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         const int zero[2] = {0, 0};  // (a copy: complete on return, whatever stream the plan is used on)
         IMG2D_CUDA(cudaMemcpy(p->counter.p, zero, sizeof(zero), cudaMemcpyHostToDevice));
     }
-    if (p->carver && !p->rows) {
+    if (p->carver) {
         // fixed scratch: fewer persistent CTAs when their private image partials would not fit
         const size_t idx_b = (size_t)nf * nextrap * ((nx + 7) / 8 * 8) * sizeof(uint16_t) + 256;
         const size_t tab_b = ((size_t)nk * ((p->L + 1) / 2 * 2) * sizeof(cpx) + 256) * (mode == OP_TWO ? 2 : 1);
