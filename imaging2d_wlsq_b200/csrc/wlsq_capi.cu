@@ -2425,7 +2425,8 @@ size_t img2d_plan_workspace_bytes(const img2d_plan *p)
 {
     if (!p) return 0;
     return p->items.bytes + p->groups.bytes + p->segs.bytes + p->owner.bytes + p->shot_off.bytes +
-           p->idx.bytes + p->tabF.bytes + p->tabB.bytes + p->tab16buf.bytes + p->partial.bytes + p->comp.bytes + p->counter.bytes +
+           p->idx.bytes + p->tabF.bytes + p->tabB.bytes + p->tab16buf.bytes + p->tab_rows.bytes + p->partial.bytes +
+           p->comp.bytes + p->visits.bytes + p->counter.bytes +
            p->naive_buf.bytes + p->adj_items.bytes + p->adj_groups.bytes + p->adj_segs.bytes + p->adj_owner.bytes +
            p->adj_work.bytes + p->adj_counter.bytes + p->adj_cache.bytes;
 }

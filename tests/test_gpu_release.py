@@ -1,4 +1,4 @@
-"""Blocks of closed plans: kept for the next plan, given back on request."""
+"""Blocks of closed plans: kept for the next plan, given back on request; the bytes a plan says it holds."""
 import pytest
 
 from imaging2d_wlsq_b200 import migration, synthetic
@@ -27,3 +27,11 @@ def test_blocks_of_closed_plans_are_reused_and_given_back():
     plan.close()
     migration.release_cached_memory()
     assert start - free() <= 4 << 20
+
+
+def test_workspace_counts_the_row_split_table():
+    """50000 rows of 31 taps: 12.8 MB in the plan's order and as much in the row-split kernel's."""
+    plan = migration.Plan(1, 4, 4, 128, 4, 4, 15, 50000)
+    assert plan.describe()["kernel"] == "migrate_rows"
+    assert plan.workspace_bytes >= 2 * 50000 * 32 * 8
+    plan.close()
