@@ -239,6 +239,11 @@ def run_reference_impl(args):
     if rank != 0:
         return 0
     from imaging2d_wlsq_b200 import synthetic
+    from oracle import oracle
+    if not oracle.have_ref():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's CPU library (oracle/_ref/extrapolation_cpu.so) "
+                                                             "is not built: its sources are not on this machine"}), flush=True)
+        return 0
     world = int(os.environ.get("WORLD_SIZE", "1"))
     maker = synthetic.WORKLOADS[args.workload]
     over = {k: v for k, v in (("nz", args.nz), ("nf", args.nf)) if v}

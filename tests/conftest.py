@@ -16,6 +16,17 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: larger CPU cases")
 
 
+def pytest_collection_modifyitems(items):
+    """The reference arm's line holds a measurement of the reference's own library: skipped, like the other
+    tests that run that library, where it is not built."""
+    from oracle import oracle
+    if oracle.have_ref():
+        return
+    for item in items:
+        if item.name == "test_reference_arm_prints_one_json_line":
+            item.add_marker(pytest.mark.skip(reason="oracle/_ref/extrapolation_cpu.so not built"))
+
+
 def rel_l2(a, b):
     """||a - b|| / ||b|| over all entries (complex entries compared as complex numbers)."""
     a = np.asarray(a)
