@@ -1242,25 +1242,26 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                              : 0;
         want_wide = p->n_slots < 12 || busy < nsm * 96 / 100;
     }
-    // The row-split kernel instead: always for a table pair and for fewer than 6 slots, else where it is
-    // estimated faster than the kernel chosen below.  Surveys of 12 slots or more are only considered
-    // when its items fill the SMs, with fewer than 16 frequencies (the least the estimates below are
-    // fitted to) four times over.
+    // The row-split kernel instead: always for a table pair and for fewer than 6 slots, else where either of
+    // two estimates finds it faster than the kernel chosen below.  Its results are the nearer ones to 64
+    // bits (four short sums per output in place of a long one: 2.6e-7 and 5.3e-7 on the gradient of 168
+    // ragged shots, 35 taps), so one of the two is enough.  Surveys of 12 slots or more are only
+    // considered when its items fill the SMs (the estimates are made for that).
     int rows_G = 1;
     std::vector<int> rows_W;  // its items' windows
     // Its CTAs have a partial image and compensation each.  Those of several CTAs per SM take at most 8 GB:
     // 5 shots of 600 traces over 4096 x 1000, 256 frequencies, took 14.5 GB.
     const int rows_most = (int)std::max<size_t>(1, (8ull << 30) / ((size_t)nsm * nextrap * nx * 8));
     RowsLaunch rows_l{1, 1e30};
+    int rows_smem_sm = 0;
     if (mode != OP_DENSE && !explicit_kernel && find_rows(1, p->L, mode == OP_TWO)) {
-        int smem_sm = 0;
-        IMG2D_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+        IMG2D_CUDA(cudaDeviceGetAttribute(&rows_smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
         for (int G = 1; G <= std::min(2, p->n_slots); ++G) {
             const int widest = make_groups(G);
             if (rows_smem_bytes(G, widest, p->L) + static_reserve > (size_t)smem_optin) continue;
             const long long n = (long long)groups.size() * nf;
-            if (p->n_slots >= 12 && mode == OP_CONJ && n < nsm * (nf < 16 ? 4 : 1)) continue;
-            const RowsLaunch r = rows_launch(G, widest, p->L, mode == OP_TWO, n, nsm, smem_sm, rows_most);
+            if (p->n_slots >= 12 && mode == OP_CONJ && n < nsm) continue;
+            const RowsLaunch r = rows_launch(G, widest, p->L, mode == OP_TWO, n, nsm, rows_smem_sm, rows_most);
             if (r.us < rows_l.us) {
                 rows_l = r;
                 rows_G = G;
@@ -1268,7 +1269,25 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                 for (const GroupDesc &g : groups) rows_W.push_back(g.W);
             }
         }
-        p->rows = rows_l.us < 1e30 && (mode == OP_TWO || p->n_slots < 6);
+        if (rows_l.us < 1e30) {
+            if (mode == OP_TWO || p->n_slots < 6) {
+                p->rows = true;
+            } else {
+                // By waves of the widest window of a line packing.  Time of a depth step of the wide kernel (8
+                // slots x up to 1024 positions per CTA) or of the 16-slot one (up to 512), in
+                // microseconds, for a CTA with all warps busy.  Clusters of three and more leave about
+                // 9% of the SMs idle.
+                const bool wide = want_wide;
+                const int G = wide ? WideShape::G : 16, pc = wide ? WideShape::PC : 512;
+                const int widest = make_groups(G), K = (widest + pc - 1) / pc;
+                const int nc = std::min(pc, (widest + K * 256 - 1) / (K * 256) * 256);
+                const double item = wide ? 0.344 * (p->L + 15) * wide_item_cost(nc, 1)
+                                         : 0.375 * (p->L + 7.4) * (nc == pc ? 1.0 : 0.57);
+                const int clusters = std::max(1, (K > 2 ? nsm * 91 / 100 : nsm) / K);
+                const double waves = (double)groups.size() * nf / clusters;
+                p->rows = 1.08 * rows_l.us < item * (waves <= 4.0 ? std::ceil(waves) : waves + 0.5);
+            }
+        }
     }
     // The 16-slot default: the wide kernel's step with 8 lanes per group (16 slots x 512 positions per
     // CTA, clusters as cluster2's), reported as the cluster2 variant after those of the table.
@@ -1322,18 +1341,14 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         }
     }
     if (!p->rows && rows_l.us < 1e30 && !p->cluster) p->rows = true;  // a lane per output: two to six times slower
-    if (!p->rows && rows_l.us < 1e30) {
+    if (!p->rows && rows_l.us < 1e30 && nf >= 16) {
         // Either kernel's items, widest first, through the queue of its CTAs or clusters.  Microseconds per
         // depth step and item, fitted on a B200 to 316 surveys of 6 to 256 shots, 16 to 256 frequencies,
         // 100 to 4096 positions, 19 to 55 taps: the wide kernel (8 slots) and the 16-slot one within 4%
-        // (standard deviation), the row-split one within 5 (a slot) and 6.5% (two).  Two of the
-        // surveys come out slower than without the row-split kernel, by 4 and 5%; taken in waves of
-        // the widest window it was twelve, by up to 19%.
-        const KernelFn rfn = find_rows(rows_G, p->L, mode == OP_TWO);
-        const size_t rsmem = rows_smem_bytes(rows_G, *std::max_element(rows_W.begin(), rows_W.end()), p->L);
-        int per_sm = 0;
-        IMG2D_CUDA(cudaFuncSetAttribute(rfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsmem));
-        IMG2D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rfn, 32 * rows_l.warps, rsmem));
+        // (standard deviation), the row-split one within 5 (a slot) and 6.5% (two).  14 of the surveys
+        // take the row-split kernel by this estimate only, 8 of 3997 traces 1.27 times as fast.
+        const size_t rsmem = rows_smem_bytes(rows_G, *std::max_element(rows_W.begin(), rows_W.end()), p->L) + 1024;
+        const int per_sm = (int)std::min<size_t>(16 / rows_l.warps, rows_smem_sm / rsmem);  // 128 registers a thread
         const int slots = (int)std::min<long long>((long long)rows_W.size() * nf, (long long)nsm * std::max(std::min(per_sm, rows_most), 1));
         const int per = (slots + nsm - 1) / nsm;  // CTAs that share an SM
         const int q = rows_np(p->L);

@@ -1,5 +1,5 @@
 """The default kernel of surveys for which either the row-split or the wide kernel is faster by 15% or more
-(measured on a B200), the ragged ones packed by windows."""
+(measured on a B200)."""
 import numpy as np
 import pytest
 
@@ -9,8 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("ns,nx,nf,taps,lo,kernel", [
-    (17, 946, 233, 25, 118, "migrate_wide"),       # 3.08 ms for 80 depth steps, row-split 3.79
-    (87, 979, 145, 25, 0, "migrate_cluster2"),     # 11.0, 16.6
+    (87, 979, 145, 25, 0, "migrate_cluster2"),     # 11.0 ms for 80 depth steps, row-split 16.6
     (7, 1741, 50, 35, 0, "migrate_wide"),          # 1.47, 1.91
     (8, 3997, 73, 25, 499, "migrate_rows"),        # the wide kernel takes 1.27 times as long
     (161, 695, 27, 25, 86, "migrate_rows"),        # 1.17 times
