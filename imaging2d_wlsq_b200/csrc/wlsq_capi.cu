@@ -2628,10 +2628,10 @@ static std::map<int, FrontScratch> g_front;
 // multiply-adds per trace; none (N1 = 0) where that exceeds 150 nt (a prime nt: cuFFT is taken) or the
 // inner sums of 8 traces do not fit in shared memory.  16 traces per CTA (64-byte reads) unless only 8
 // leave room for two CTAs per SM.
-static SpecPlan spec_plan(int nt, int nf, size_t smem_optin)
+static SpecPlan spec_plan(int nt, int nf, size_t smem_optin, double &best_cost)
 {
     SpecPlan best{};
-    double best_cost = 150.0 * nt;
+    best_cost = 150.0 * nt;
     for (int N1 = 1; N1 <= 31 && N1 <= nt; ++N1) {
         if (nt % N1) continue;
       for (int M : {8, 10}) {
@@ -2655,37 +2655,19 @@ static SpecPlan spec_plan(int nt, int nf, size_t smem_optin)
         }
       }
     }
+    // a few tasks in the second stage: their sums in parts of whole blocks, as many as there are threads for
+    // and as the inner sums' place holds partial sums
+    best.S = 1;
+    best.T2 = best.N2;
+    if (best.N1) {
+        const int tasks = std::min(best.N1, nf) * (best.mp / best.M);
+        const int parts = std::min(256 / (best.C / 2) / tasks, best.N2 * best.K1 / (tasks * best.M));
+        if (parts >= 4) {
+            best.T2 = ((best.N2 + parts - 1) / parts + kSpecBlock - 1) / kSpecBlock * kSpecBlock;
+            best.S = (best.N2 + best.T2 - 1) / best.T2;
+        }
+    }
     return best;
-}
-
-// Time of the two-stage transform and of the library's in microseconds, within 25% of what 150 calls took on
-// a B200 (1 to 62 shots of 100 to 2000 traces, 300 to 3000 samples, 16 to 1700 rows).
-//
-// Ours: CTAs in waves, each the iterations of its tasks' two loops.  With few residues (N1 small: nt a
-// prime times 1 to 4) there are fewer tasks than threads for them and the second loop, N2 long,
-// is waited for: 25 shots of 716 traces, 1553 samples, 20 rows 4.0 ms against 0.73.
-static double spec_us(const SpecPlan &pl, int nf, const std::vector<int> &w, int nsm, int smem_sm)
-{
-    long long ctas = 0;
-    for (int x : w) ctas += (x + pl.C - 1) / pl.C;
-    const int room = nsm * std::max(1, std::min(2, smem_sm / (int)(pl.smem + 3072)));
-    const double waves = ctas < 4ll * room ? (double)((ctas + room - 1) / room) : (double)ctas / room + 0.5;
-    auto rounds = [](int tasks, int threads) { return (tasks + 256 / threads - 1) / (256 / threads); };
-    const int first = rounds((pl.N2 + kSpecT - 1) / kSpecT * ((pl.K1 + kSpecKC - 1) / kSpecKC), pl.C);
-    const int second = rounds(std::min(pl.N1, nf) * (pl.mp / pl.M), pl.C / 2);
-    return waves * (0.8 * first * (pl.N1 / 2 + 1) + (pl.M == 8 ? 0.27 : 0.36) * second * pl.N2);
-}
-
-// The library: all nx traces to all rows, a launch or more per shot (lengths with a prime factor above 13
-// twice the time), then the packing of the kept rows; large shots overlap with the launches.
-static double cufft_us(int ns, int nt, int nx, int nf)
-{
-    int rest = nt;
-    for (int q : {2, 3, 5, 7, 11, 13})
-        while (rest % q == 0) rest /= q;
-    const double shot = 1e-6 * nt * (double)nx;
-    const double us = 45.0 + ns * ((rest == 1 ? 8.0 : 15.0) + 11.0 * shot + 9e-6 * nf * (double)nx);
-    return shot >= 1.0 ? std::min(us, 500.0 + 8.5 * ns * shot) : us;
 }
 
 static SpecShots spec_shots(int s0, int n, const std::vector<int> &x0, const std::vector<int> &w,
@@ -2773,22 +2755,28 @@ int img2d_records_to_spectra(int ns, int nt, int nx, int nf, int nt_rows, const 
     if ((rc = spectra_layout(ns, nt, nx, nf, nt_rows, shot_x0, shot_nx, x0, w, off))) return rc;
     if (!d_records || !d_out) return fail(IMG2D_EINVAL, "null pointer argument");
     cudaStream_t st = (cudaStream_t)stream;
-    int dev = 0, smem_optin = 0, smem_sm = 0, nsm = 0;
+    int dev = 0, smem_optin = 0;
     IMG2D_CUDA(cudaGetDevice(&dev));
     IMG2D_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    IMG2D_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    IMG2D_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     std::lock_guard<std::mutex> lock(g_front_mu);
     FrontScratch &fs = g_front[dev];
-    const SpecPlan pl = spec_plan(nt, nf, (size_t)smem_optin);
-    if (!pl.N1 || spec_us(pl, nf, w, nsm, smem_sm) > cufft_us(ns, nt, nx, nf))
-        return spectra_by_cufft(fs, ns, nt, nx, nf, d_records, x0, w, off, (cpx *)d_out, st);
+    double cost;
+    const SpecPlan pl = spec_plan(nt, nf, (size_t)smem_optin, cost);
+    // cuFFT transforms all nx traces to all rows: about 0.5 ms of launches and 8.5 ps per sample.  It
+    // is the faster one where most rows of many full-width records are kept (256 x 1024 x 2048 samples
+    // to 512 rows: 6.0 ms here, 5.0 ms with cuFFT; 32 x 1024 x 1024 to 512 rows: 0.43 and 1.0 ms).
+    double traces = 0.0;
+    for (int x : w) traces += x;
+    const bool library = 8.2e-11 * cost * traces > 0.5 + 8.5e-9 * ns * nt * (double)nx;
+    if (!pl.N1 || library) return spectra_by_cufft(fs, ns, nt, nx, nf, d_records, x0, w, off, (cpx *)d_out, st);
     const size_t n1 = (size_t)kSpecK * kSpecK, n2 = (size_t)pl.N2 * pl.mp, n3 = (size_t)nt;
     if ((rc = fs.tables.ensure((n1 + n2 + n3) * sizeof(float2)))) return rc;
     float2 *T1 = fs.tables.as<float2>(), *B = T1 + n1, *A = B + n2;
     spec_tables_kernel<<<(int)std::min<size_t>((n1 + n2 + n3 + 255) / 256, 148 * 4), 256, 0, st>>>(pl, nt, T1, B, A);
     IMG2D_CUDA(cudaGetLastError());
-#define IMG2D_SPEC(C, M) (pl.bs ? record_spectra_kernel<C, M, true> : record_spectra_kernel<C, M, false>)
+#define IMG2D_SPEC(C, M)                                                                                       \
+    (pl.S > 1 ? (pl.bs ? record_spectra_kernel<C, M, true, true> : record_spectra_kernel<C, M, false, true>)   \
+              : (pl.bs ? record_spectra_kernel<C, M, true, false> : record_spectra_kernel<C, M, false, false>))
     auto kernel = pl.C == 16 ? (pl.M == 8 ? IMG2D_SPEC(16, 8) : IMG2D_SPEC(16, 10))
                              : (pl.M == 8 ? IMG2D_SPEC(8, 8) : IMG2D_SPEC(8, 10));
 #undef IMG2D_SPEC

@@ -17,8 +17,8 @@
 //            shared memory, single precision like the reference's transform of float32 records;
 //   sources  source_spectra_kernel: a Ricker wavelet sampled in float32 is exactly zero away from its
 //            arrival, so its spectrum is a short sum and the time-domain array is never formed.
-// Lengths without a divisor that makes the first worthwhile (primes), and calls that spec_us and
-// cufft_us estimate to be faster there (few residues, or most rows of large records), go through cuFFT, one
+// Lengths without a divisor that makes the first worthwhile (primes), and most rows of many large
+// records, go through cuFFT, one
 // real-to-complex transform per shot, and pack_spectra_kernel.
 //
 // Measured on a B200, 32 shots of 1500 x 1024 samples, 256 rows, sources and records: 2.33 ms with
@@ -112,6 +112,7 @@ constexpr int kSpecT = 4;     // values of t2 per task
 constexpr int kSpecBlock = 8; // terms of a partial sum of the second stage
 struct SpecPlan {
     int N1, N2, K1, mp, C, M;  // C: traces per CTA, M: outer outputs per thread and pass
+    int S, T2;                     // second stage: parts of the sum over t2 (1: whole sums), terms of a part
     bool bs;                       // table B in shared memory
     size_t smem;
 };
@@ -143,7 +144,10 @@ __global__ void spec_tables_kernel(SpecPlan pl, int nt, float2 *__restrict__ T1,
 //            memory (BS, up to 8 KB: one load from L2 per factor was waited for 50 times).  Sums of 8 terms, then their sum: with one running sum over N2 = 50 terms the error
 //            against 64 bits was 2.1e-7, cuFFT's 1.6e-7.
 // One trace per thread and 8 per load: 446 us for 32 shots of 1500 x 1024 samples, 256 rows.
-template <int C, int M, bool BS>
+// SPLIT: lengths with few residues (a large prime times 1 to 4) have a few tasks of very long sums.  Their
+// sums over t2 are shared out over the idle threads in S parts, added in order at the end: 25
+// shots of 1553 x 716 samples, 20 rows, with their sources 4.0 ms without, 0.42 with (cuFFT 0.73).
+template <int C, int M, bool BS, bool SPLIT>
 __global__ void __launch_bounds__(256, 2) record_spectra_kernel(SpecPlan pl, SpecShots sh, int s0, int nt, int nx,
                                                                 int nf, const float *__restrict__ rec,
                                                                 const float2 *__restrict__ T1,
@@ -213,23 +217,21 @@ __global__ void __launch_bounds__(256, 2) record_spectra_kernel(SpecPlan pl, Spe
     __syncthreads();
     constexpr int H = C / 2;  // threads per task; traces col and col + H
     const int col = threadIdx.x % H;
-    const int nm = pl.mp / M;
-    for (int task = threadIdx.x / H; task < min(N1, nf) * nm; task += 256 / H) {
-        const int k1 = task / nm, m0 = task % nm * M;
-        if (k1 + N1 * m0 >= nf) continue;
+    const int nm = pl.mp / M, tasks = min(N1, nf) * nm;
+    // sums of outputs k1 + N1 (m0 + m) over t2 in [first, last)
+    auto sum = [&](int k1, int m0, int first, int last, float (&sre)[2][M], float (&sim)[2][M]) {
         const bool conj = k1 >= K1;
         const float2 *y = Y + (conj ? N1 - k1 : k1) * C + col;
         const float4 *w = BS ? Bs + m0 / 2 : reinterpret_cast<const float4 *>(B + m0);
         const float2 *turn = A + (long long)k1 * N2;
-        float sre[2][M], sim[2][M];
 #pragma unroll
         for (int m = 0; m < M; ++m) sre[0][m] = sim[0][m] = sre[1][m] = sim[1][m] = 0.f;
-        for (int tb = 0; tb < N2; tb += kSpecBlock) {
+        for (int tb = first; tb < last; tb += kSpecBlock) {
             float re[2][M], im[2][M];
 #pragma unroll
             for (int m = 0; m < M; ++m) re[0][m] = im[0][m] = re[1][m] = im[1][m] = 0.f;
 #pragma unroll 2
-            for (int t2 = tb; t2 < min(tb + kSpecBlock, N2); ++t2) {
+            for (int t2 = tb; t2 < min(tb + kSpecBlock, last); ++t2) {
                 float2 v[2] = {y[t2 * K1 * C], y[t2 * K1 * C + H]};
                 const float2 q = __ldg(turn + t2);
 #pragma unroll
@@ -262,6 +264,8 @@ __global__ void __launch_bounds__(256, 2) record_spectra_kernel(SpecPlan pl, Spe
                     sim[i][m] += im[i][m];
                 }
         }
+    };
+    auto store = [&](int k1, int m0, const float (&sre)[2][M], const float (&sim)[2][M]) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int x = x0 + col + i * H;
@@ -273,6 +277,40 @@ __global__ void __launch_bounds__(256, 2) record_spectra_kernel(SpecPlan pl, Spe
                 if (k < nf) o[(long long)k * ws] = cpx{sre[i][m], sim[i][m]};
             }
         }
+    };
+    float sre[2][M], sim[2][M];
+    if (!SPLIT) {
+        for (int task = threadIdx.x / H; task < tasks; task += 256 / H) {
+            const int k1 = task / nm, m0 = task % nm * M;
+            if (k1 + N1 * m0 >= nf) continue;
+            sum(k1, m0, 0, N2, sre, sim);
+            store(k1, m0, sre, sim);
+        }
+        return;
+    }
+    // S tasks <= 256 / H: one part a thread
+    const int part = threadIdx.x / H / tasks, task = threadIdx.x / H % tasks;
+    const int k1 = task / nm, m0 = task % nm * M;
+    const bool active = part < pl.S && k1 + N1 * m0 < nf;
+    if (active) sum(k1, m0, part * pl.T2, min((part + 1) * pl.T2, N2), sre, sim);
+    __syncthreads();
+    float2 *const P = Y;  // [part][task][2 M][H], once Y has been read
+    if (active && part > 0) {
+#pragma unroll
+        for (int e = 0; e < 2 * M; ++e)
+            P[((part * tasks + task) * 2 * M + e) * H + col] = make_float2(sre[e / M][e % M], sim[e / M][e % M]);
+    }
+    __syncthreads();
+    if (active && part == 0) {
+        for (int r = 1; r < pl.S; ++r) {
+#pragma unroll
+            for (int e = 0; e < 2 * M; ++e) {
+                const float2 v = P[((r * tasks + task) * 2 * M + e) * H + col];
+                sre[e / M][e % M] += v.x;
+                sim[e / M][e % M] += v.y;
+            }
+        }
+        store(k1, m0, sre, sim);
     }
 }
 
