@@ -727,7 +727,8 @@ struct img2d_plan {
     // demigration (adjoint) launch state, built on its first call
     int adj_G = 0, adj_grid = 0, adj_items_n = 0, adj_wmax = 0, adj_block = 0, adj_slab = 0, adj_nslab = 0;
     int adj_cluster = 0;               // CTAs per cluster of the cluster demigration kernel, 0 = single CTA
-    bool adj_rows = false, adj_allow_rows = true, adj_allow_wide = true;  // the row-split demigration kernel
+    bool adj_rows = false;             // the row-split demigration kernel
+    bool adj_allow_rows = true, adj_allow_wide = true;  // until their planes did not fit in memory
     void (*adj_rows_fn)(img2d::RowsAdjArgs) = nullptr;
     void (*adj_wide_fn)(img2d::DemigrateArgs, int *) = nullptr;  // the wide demigration kernel
     bool adj_full_cache = false;       // kept source: every depth step of every item (else per-CTA planes only)
@@ -1113,11 +1114,13 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
     std::vector<int16_t> owner;
     auto make_groups = [&](int G) { return pack_groups(p, G, groups, segs, owner); };
 
-    // Kernel choice.  The second-generation cluster kernel (16 slots per item, 512 positions per CTA,
-    // clusters of up to 16 CTAs where they fit) when there are enough slots to fill it and the
-    // operator has at least 7 taps; else the first-generation cluster kernel (256 positions per CTA,
-    // up to 8 CTAs, compile-time operator lengths); otherwise the single-CTA kernels with the
-    // largest power of two <= 8 slots whose ping-pong buffers fit in shared memory.
+    // Kernel choice, for 7 taps and more.  8 slots: the wide kernel (try_wide) where the 16-slot kernels'
+    // clusters would leave SMs idle or there are 6 to 11 slots.  16 slots: the same kernel with 8 lanes
+    // per group (try_wide16, up to 65 taps), else the second-generation cluster kernel, else the
+    // first-generation one (256 positions per CTA, up to 8 CTAs, compile-time lengths).  The row-split
+    // kernel for table pairs, fewer than 6 slots, and where it is estimated faster than any of these.
+    // Otherwise the single-CTA kernels with the largest power of two <= 8 slots whose ping-pong
+    // buffers fit in shared memory.
     p->cluster = 0;
     p->block = 256;
     const bool cluster_ok = mode == OP_CONJ && !(flags & (IMG2D_FLAG_GENERIC | IMG2D_FLAG_NO_CLUSTER)) &&
@@ -1345,8 +1348,8 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
         // Either kernel's items, widest first, through the queue of its CTAs or clusters.  Microseconds per
         // depth step and item, fitted on a B200 to 316 surveys of 6 to 256 shots, 16 to 256 frequencies,
         // 100 to 4096 positions, 19 to 55 taps: the wide kernel (8 slots) and the 16-slot one within 4%
-        // (standard deviation), the row-split one within 5 (a slot) and 6.5% (two).  14 of the surveys
-        // take the row-split kernel by this estimate only, 8 of 3997 traces 1.27 times as fast.
+        // (standard deviation), the row-split one within 5 (a slot) and 6.5% (two), which is the margin.
+        // 8 of the surveys take the row-split kernel by this estimate only, 3 to 27% faster.
         const size_t rsmem = rows_smem_bytes(rows_G, *std::max_element(rows_W.begin(), rows_W.end()), p->L) + 1024;
         const int per_sm = (int)std::min<size_t>(16 / rows_l.warps, rows_smem_sm / rsmem);  // 128 registers a thread
         const int slots = (int)std::min<long long>((long long)rows_W.size() * nf, (long long)nsm * std::max(std::min(per_sm, rows_most), 1));
@@ -1371,7 +1374,7 @@ static int build_plan(img2d_plan *p, int ns, int nextrap, int nz, int nx, int nf
                                  : 1.5 + 0.02 * p->L + (0.85 + 0.35 * p->L) * share);
         }
         const int clusters = std::max(1, clusters_that_fit((const void *)p->fn, K, p->block, p->smem));
-        p->rows = queue_time(mine, nf, slots) < queue_time(other, nf, clusters);
+        p->rows = 1.06 * queue_time(mine, nf, slots) < queue_time(other, nf, clusters);
     }
     if (p->rows) {
         p->cluster = 0;
