@@ -95,8 +95,9 @@ __host__ __device__ inline size_t wide_bulk_smem_bytes(int M, bool stage)
     return wide_bulk_bar_offset(M, stage) + (size_t)WideShape::NW * 2 * sizeof(unsigned long long);
 }
 
-// SM clock cycles (about a second) after which a ring-chunk wait gives up: the thread then records
-// the failure in the launch's status word and neither waits for nor issues ring chunks again, so a
+// SM clock cycles (1.1 s) after which a ring-chunk wait gives up (waits for neighbours allow twice as
+// many): the thread then records
+// the failure in the plan's status word and neither waits for nor issues ring chunks again, so a
 // phase that can never complete ends the launch instead of hanging it.
 constexpr long long kBulkWaitCycles = 1ll << 31;
 

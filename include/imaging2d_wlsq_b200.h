@@ -51,9 +51,11 @@ typedef struct {
  * lines across the model, lines grouped by extent) instead of the window-first packing, which the
  * plan otherwise uses where its modelled cost is lower */
 #define IMG2D_FLAG_LINE_PACKING (1 << 19)
-/* Default kernel choice: the wide cluster kernel where the 16-slot kernel's clusters would leave
- * SMs idle (or fewer than 12 lane slots), else the 16-slot cluster kernel; the single-CTA kernels
- * for fewer than 6 lane slots, operators shorter than 7 taps or windows beyond 16 CTAs. */
+/* Default kernel choice: the row-split kernel for two tables, for fewer than 6 lane slots and for
+ * surveys estimated to be faster that way (3 to 79 taps, windows that fit one CTA); else the wide
+ * cluster kernel where the 16-slot kernel's clusters would leave SMs idle (or fewer than 12 lane
+ * slots), else the 16-slot cluster kernel; the single-CTA kernels for the rest (windows beyond 16
+ * CTAs, lengths that none of these takes). */
 /* select variant v (1-based; 0 = default) of the second-generation cluster kernel: bits 8-15 */
 #define IMG2D_FLAG_VARIANT_SHIFT 8
 #define IMG2D_FLAG_VARIANT(v) ((v) << IMG2D_FLAG_VARIANT_SHIFT)
@@ -255,7 +257,8 @@ int img2d_migrate_compact_noalloc(int ns, int nextrap, int nz, int nx, int nf, i
  * computes d_data = F* m for the reflectivity m = d_refl (rows [0, nextrap) of an nx-wide float
  * image), with <F d, m> = Re sum d conj(F* m).  It sweeps the depth steps in reverse order with
  * the transposed operators and recomputes the source wavefield per slab of slab_depth steps from
- * checkpoints (slab_depth <= 0: 8).  Writes rows [0, nf) of every shot block of d_data (packed like
+ * checkpoints (slab_depth <= 0: 8; with fewer than 12 lane slots every step is kept instead,
+ * where memory allows, and slab_depth has no effect).  Writes rows [0, nf) of every shot block of d_data (packed like
  * d_wave, must not alias it).  Single-table mode only (T_back = conj(T_forw)); uses the FP32 table.
  * Asynchronous on `stream`; img2d_plan_kernel_ms then times this kernel.
  *
@@ -263,10 +266,13 @@ int img2d_migrate_compact_noalloc(int ns, int nextrap, int nz, int nx, int nf, i
  * demigrations with the same source (a least-squares migration loop) can keep its checkpoints.
  *   IMG2D_SOURCE_RECOMPUTE  checkpoints in per-CTA scratch, recomputed by this call, not kept;
  *   IMG2D_SOURCE_KEEP       checkpoints computed by this call and kept on the plan
- *                           (items x slabs x window x slots x 8 bytes of device memory);
+ *                           (items x slabs x window x slots x 8 bytes of device memory).  With fewer
+ *                           than 12 lane slots every depth step is kept (items x steps x window x
+ *                           slots x 8 bytes) up to 8 GB, above that nothing;
  *   IMG2D_SOURCE_REUSE      the kept checkpoints are read instead of computed (the checkpoint pass,
- *                           a third of the work, is skipped).  The caller guarantees the same
- *                           d_wave contents as the keeping call; img2d_plan_set_model and a
+ *                           a third of the work, is skipped; with every step kept all of the source's
+ *                           work, half of the whole; with nothing kept none).  The caller guarantees
+ *                           the same d_wave contents as the keeping call; img2d_plan_set_model and a
  *                           different slab_depth discard the kept checkpoints (IMG2D_EINVAL).
  * ---------------------------------------------------------------------------------------- */
 #define IMG2D_SOURCE_RECOMPUTE 0
